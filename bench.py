@@ -143,8 +143,8 @@ def survey_bytes(m_r: list, n_r: list, count: int) -> int:
 
 
 def kernel_bytes(m: int, stats) -> dict:
-    """Algorithmic bytes per solve of each kernel, from the rounds it ran: an
-    edge pass reads its input (12-byte caller records in round 0 and in the
+    """Algorithmic bytes per solve of each phase of the solve kernel, from the
+    rounds it ran, and of the kernel (their sum): an edge pass reads its input (12-byte caller records in round 0 and in the
     heavy pass, 16-byte survivor records otherwise) and writes 16 bytes per
     survivor; the hook reads best (8), the survivor record (16), the partner's
     best (8) and writes parent (4) per choosing component; the gather reads the
@@ -154,8 +154,9 @@ def kernel_bytes(m: int, stats) -> dict:
     for r, mr in enumerate(m_r):
         from_input = r == 0 or r == stats.light_rounds
         ep += (12 * m if from_input else 16 * m_r[r - 1]) + 16 * mr
-    return {"msf_edge_pass": ep, "msf_hook": 36 * sum(stats.n_r),
-            "msf_gather": (m + 31) // 32 * 4 + 24 * stats.count}
+    phases = {"msf_edge_pass": ep, "msf_hook": 36 * sum(stats.n_r),
+              "msf_gather": (m + 31) // 32 * 4 + 24 * stats.count}
+    return {"msf_solve": sum(phases.values()), **phases}
 
 
 def rounds_fixture(scale: int, edge_factor: int):
@@ -879,9 +880,6 @@ def profile_solves(args) -> None:
     import phem_graph_b200 as P
     g, E = rmat22(0, args.scale, args.edge_factor)
     ctx = P.Context(0)
-    # the rounds queued on the stream: ncu does not profile the kernel nodes
-    # of a graph that has conditional nodes
-    ctx.set_tuning("msf.graph", 0)
     d = torch.from_numpy(E.view(np.int32)).to("cuda:0")
     o = torch.empty((g.n, 3), dtype=torch.int32, device="cuda:0")
     ct = torch.zeros(2, dtype=torch.int64, device="cuda:0")
@@ -987,7 +985,7 @@ def main() -> None:
         t_ms = ev0.elapsed_time(ev1)
         launches = ctx.profile()
         # the same steps again with every launch bracketed by CUDA events on
-        # the solve's stream: per-kernel durations for the roofline
+        # the solve's stream, and the solve's phases stamped by the device
         ctx.profile_reset()
         ctx.set_profiling(True)
         with torch.cuda.stream(stream):
@@ -1037,9 +1035,11 @@ def main() -> None:
     timed = {k: v for k, v in prof.items() if v["timed_launches"]}
     dom = max(timed, key=lambda k: timed[k]["total_ms"]) if timed else None
     kernels = {}
-    total_kernel_ms = sum(v["total_ms"] for v in timed.values()) or 1.0
+    total_kernel_ms = sum(v["total_ms"] for v in timed.values() if v["launches"]) or 1.0
     for k, v in timed.items():
-        entry = {"launches": v["launches"], "ms_per_step": v["total_ms"] / args.steps,
+        # the phases of msf_solve have no launches of their own
+        entry = {"launches": v["launches"], "timed": v["timed_launches"],
+                 "ms_per_step": v["total_ms"] / args.steps,
                  "share": v["total_ms"] / total_kernel_ms}
         if k in byts:
             gbs = byts[k] * args.steps / (v["total_ms"] / 1e3) / 1e9
@@ -1048,13 +1048,13 @@ def main() -> None:
     roofline = None
     if dom:
         achieved = kernels[dom].get("achieved_gbs")
-        traffic = (profile_traffic("edge_pass", "msf_edge_pass_rmat22_dram.csv", 1)
-                   if (dom == "msf_edge_pass" and args.scale == 22 and args.edge_factor == 16) else None)
+        traffic = (profile_traffic("solve_kernel", "msf_solve_rmat22_dram.csv", 1)
+                   if (dom == "msf_solve" and args.scale == 22 and args.edge_factor == 16) else None)
         roofline = {"kernel": dom, "bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                     "frac": (achieved / peaks["hbm_gbs"]) if achieved else None,
                     "traffic": traffic,
-                    "traffic_basis": "ncu dram__bytes_read + write of the edge-pass launches of one solve "
-                                     "(profiles/msf_edge_pass_rmat22_dram.csv, bench.py --profile-solves 1)",
+                    "traffic_basis": "ncu dram__bytes_read + write of one solve's launch "
+                                     "(profiles/msf_solve_rmat22_dram.csv, bench.py --profile-solves 1)",
                     "peak_source": f"{peaks['source']} (MEASURED_PEAKS.json hbm_gbs)",
                     "algorithmic_bytes_per_step": byts.get(dom)}
     solve_gbs = byts["survey"] / (ms_per_step / 1e3) / 1e9 if byts["survey"] else None
@@ -1073,7 +1073,8 @@ def main() -> None:
         "device_rounds": {"m_r": stats.m_r, "n_r": stats.n_r, "light_rounds": stats.light_rounds,
                           "threshold_weight": stats.threshold >> 32},
         "kernels": kernels,
-        "kernel_timing": "the timed steps repeated with CUDA events around every launch on the solve's stream",
+        "kernel_timing": "the timed steps repeated with CUDA events around every launch on the solve's stream "
+                         "and the device's own timestamps between the solve's phases",
         "result": {"msf_edges": stats.count, "total_weight": stats.total, "rounds": stats.rounds},
         "e2e": {"value": world * m / e2e_s / 1e9, "unit": UNIT, "h2d_bytes_per_step": m * 12,
                 "d2h_bytes_per_step": r_host.count * 12 + 16, "ms_per_step": e2e_s * 1e3,

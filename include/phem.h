@@ -88,7 +88,10 @@ phem_status phem_context_set_timeout_ms(phem_context *ctx, uint32_t ms);
 
 /* Per-kernel accounting.  Every kernel launch is counted; with profiling on,
  * each launch is also bracketed by CUDA events on the context stream and its
- * duration added up (for roofline figures measured inside an application). */
+ * duration added up (for roofline figures measured inside an application).
+ * The MSF solve is one launch ("msf_solve"); its phases ("msf_edge_pass",
+ * "msf_hook", ...) are listed beside it with no launches of their own, timed
+ * by the device. */
 typedef struct phem_kernel_profile {
     char name[32];
     uint64_t launches;        /* launches since the last reset */
@@ -102,7 +105,8 @@ phem_status phem_context_set_profiling(phem_context *ctx, int on);
 phem_status phem_context_profile(phem_context *ctx, phem_kernel_profile *out, uint32_t max, uint32_t *count);
 phem_status phem_context_profile_reset(phem_context *ctx);
 
-/* Event-timed launches in launch order since the last reset (profiling on). */
+/* Timed launches and phases in order of completion since the last reset
+ * (profiling on). */
 typedef struct phem_launch_record {
     char name[32];
     float ms;
@@ -113,14 +117,9 @@ phem_status phem_context_launch_log(phem_context *ctx, phem_launch_record *out, 
  *   "msf.light_per_vertex"  light edges per vertex taken by the MSF filter
  *                           before the heavy pass; 0 disables the filter   [0.5]
  *   "msf.filter_min_ratio"  filter only when m >= ratio * light edges      [2.0]
- *   "msf.first_batch"       Boruvka rounds queued before the first check  [12]
- *   "msf.next_batch"        rounds queued per later check                 [4]
- *   "msf.edge_ctas_per_sm"  CTAs of 8 independent warps per SM in the edge
- *                           pass, 1 to 4                                  [4]
- *   "msf.graph"             1: the Boruvka rounds run as a cached CUDA graph
- *                           whose while-node the device drives; 0: rounds
- *                           queued on the stream in batches (per-launch
- *                           profiling always uses the stream form)        [1]
+ *   "msf.edge_ctas_per_sm"  groups of 8 warps per SM in the solve, 1 to 4 [4]
+ *   "msf.first_batch", "msf.next_batch", "msf.graph"  accepted and without
+ *                           effect: the rounds run inside one launch  [12, 4, 1]
  *   "cc.canonical_light_per_vertex"  msf.light_per_vertex for the
  *                           PHEM_CC_CANONICAL forest (light = first by index) [1.5]
  *   "cc.sample_per_vertex"  phem_cc_solve unites this many edges per vertex

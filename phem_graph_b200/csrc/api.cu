@@ -21,7 +21,7 @@ thread_local char g_last_error[512] = "";
 }  // namespace
 
 const char *const kKernelNames[kKernelCount] = {
-    "msf_init", "msf_select", "msf_edge_pass", "msf_hook", "msf_compress", "msf_advance", "msf_gather",
+    "msf_solve", "msf_init", "msf_select", "msf_edge_pass", "msf_hook", "msf_compress", "msf_gather",
     "cc_init", "cc_unite", "cc_merge", "cc_label", "cc_minid", "cc_count", "csr_to_coo", "batch_solve"};
 
 constexpr size_t kLaunchLogCap = 1u << 16;
@@ -78,6 +78,16 @@ void resolve_timings(phem_context *ctx)
         ctx->event_pool.push_back(p.stop);
     }
     ctx->pending.clear();
+}
+
+void log_phase(phem_context *ctx, int kernel, float ms)
+{
+    if (kernel < 0 || kernel >= kKernelCount)
+        return;
+    ctx->kernel_ms[kernel] += ms;
+    ctx->timed_launches[kernel]++;
+    if (ctx->launch_log.size() < kLaunchLogCap)
+        ctx->launch_log.emplace_back(kernel, ms);
 }
 
 void set_error(const char *fmt, ...)
@@ -306,9 +316,6 @@ void phem_context_destroy(phem_context *ctx)
     DeviceGuard g(ctx->device);
     if (ctx->stream)
         cudaStreamSynchronize(ctx->stream);
-    for (auto &e : ctx->msf_exec)
-        if (e)
-            cudaGraphExecDestroy(e);
     if (ctx->ws)
         cudaFree(ctx->ws);
     if (ctx->input)
@@ -381,7 +388,7 @@ phem_status phem_context_profile(phem_context *ctx, phem_kernel_profile *out, ui
     resolve_timings(ctx);
     uint32_t k = 0;
     for (int i = 0; i < kKernelCount; i++) {
-        if (!ctx->launches[i])
+        if (!ctx->launches[i] && !ctx->timed_launches[i])
             continue;
         if (out && k < max) {
             std::memset(&out[k], 0, sizeof(out[k]));
@@ -601,7 +608,7 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
     size_t base = 0;
     MsfPlan plan;
     if (canonical) {
-        PHEM_TRY(msf_plan(ctx, kKindPacked, nullptr, (uint64_t)m, (uint32_t)n, extra, &plan, &base));
+        PHEM_TRY(msf_plan(ctx, nullptr, (uint64_t)m, (uint32_t)n, extra, &plan, &base));
     } else {
         PHEM_TRY(ws_reserve(ctx, extra));
     }
@@ -629,7 +636,7 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
     if (canonical) {
         plan.e0 = d_edges;
         plan.forest = d_for;
-        PHEM_TRY(msf_run(ctx, kKindPacked, plan, &rounds));
+        PHEM_TRY(msf_run(ctx, kKindPacked, plan));
         // plan.best is free after the rounds: reuse it as the per-root min-id array
         PHEM_TRY(cc_launch_minid_labels(ctx, n, plan.parent, reinterpret_cast<uint32_t *>(plan.best), d_lab));
     } else {
@@ -653,14 +660,14 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
         }
         PHEM_TRY(cc_launch_label(ctx, n, d_par, d_lab));
     }
-    const float ms = timer.stop();
-    PHEM_CUDA_TRY(cudaMemsetAsync(&ctx->ctl->misc[0], 0, 2 * sizeof(unsigned long long), ctx->stream));
+    cudaEventRecord(ctx->ev_stop, ctx->stream);
     PHEM_TRY(cc_launch_count(ctx, n, d_lab, d_for));
     PHEM_TRY(copy_back(ctx, sl, lb));
     PHEM_TRY(copy_back(ctx, sf, fb));
-    PHEM_CUDA_TRY(cudaMemcpyAsync(ctx->h_ctl, ctx->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, ctx->stream));
-    PHEM_TRY(stream_wait(ctx));
-    PHEM_TRY(ctl_status(ctx->h_ctl->err, "cc_solve"));
+    PHEM_TRY(msf_finish(ctx, &rounds, "cc_solve"));
+    float ms = 0.f;
+    if (cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop) != cudaSuccess)
+        ms = 0.f;
     if (stats) {
         stats->components = (uint32_t)ctx->h_ctl->misc[0];
         stats->forest_edges = d_for ? ctx->h_ctl->misc[1] : (uint64_t)n - ctx->h_ctl->misc[0];
@@ -922,7 +929,7 @@ static phem_status msf_common(phem_context *ctx, const phem_edge *edges, uint64_
     const size_t o_edges = 0, o_out = aligned_dev ? 0 : align256(eb);  // edges read in place: no staging area
     size_t base = 0;
     MsfPlan plan;
-    PHEM_TRY(msf_plan(ctx, kKindMsf, nullptr, m, n, o_out + align256(ob), &plan, &base));
+    PHEM_TRY(msf_plan(ctx, nullptr, m, n, o_out + align256(ob), &plan, &base));
     Staged se, so;
     if (aligned_dev) {
         se.dev = const_cast<phem_edge *>(edges);
@@ -933,22 +940,20 @@ static phem_status msf_common(phem_context *ctx, const phem_edge *edges, uint64_
     }
     stage_out(ctx, msf, ob, base + o_out, &so);
     plan.e0 = se.dev;
+    plan.out = static_cast<phem_edge *>(so.dev);
+    plan.gather = 1;
     Timed timer(ctx);
     uint32_t rounds = 0;
-    // rounds, gather and the count copy are queued back to back; one wait at
-    // the end (a host round trip between them would leave the GPU idle)
-    PHEM_TRY(msf_run(ctx, kKindMsf, plan, &rounds, true));
-    PHEM_TRY(msf_gather(ctx, plan, static_cast<phem_edge *>(so.dev)));
+    PHEM_TRY(msf_run(ctx, kKindMsf, plan));
     PHEM_CUDA_TRY(cudaEventRecord(ctx->ev_stop, ctx->stream));
     if (d_count_total)
         PHEM_CUDA_TRY(cudaMemcpyAsync(d_count_total, &ctx->ctl->msf_count, 2 * sizeof(uint64_t),
                                       cudaMemcpyDeviceToDevice, ctx->stream));
-    PHEM_TRY(msf_finish(ctx, &rounds));
+    PHEM_TRY(msf_finish(ctx, &rounds, "msf"));
     float ms = 0.f;
     if (cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop) != cudaSuccess)
         ms = 0.f;
     const Ctl &h = *ctx->h_ctl;
-    PHEM_TRY(ctl_status(h.err, "msf"));
     if (h.msf_count > (uint64_t)n - 1 + (n == 0)) {
         set_error("msf: %llu forest edges for %u vertices", (unsigned long long)h.msf_count, n);
         return PHEM_ERR_NONCONVERGED;
@@ -1067,7 +1072,7 @@ static phem_status msf_stream_impl(phem_context *ctx, const phem_edge *h_edges, 
         // size the solve workspace once for the largest solve (a later growth
         // would free memory, which waits for the copies in flight)
         MsfPlan plan;
-        PHEM_TRY(msf_plan(ctx, kKindMsf, nullptr, R + top, n, align256((size_t)n * sizeof(phem_edge)), &plan,
+        PHEM_TRY(msf_plan(ctx, nullptr, R + top, n, align256((size_t)n * sizeof(phem_edge)), &plan,
                           nullptr));
     }
     char *b = static_cast<char *>(ctx->input);

@@ -24,40 +24,36 @@ constexpr uint64_t kKeyNone = ~0ull;           // "no candidate edge" (w = id = 
 constexpr uint64_t kForestEmpty = 0x7fffffffull;
 constexpr int kBlock = 256;                    // threads per block for the streaming kernels
 constexpr int kWarps = kBlock / 32;
-constexpr int kItems = 4;                      // records per thread per tile
-constexpr int kTile = kBlock * kItems;         // records per tile
 constexpr uint32_t kUnionRetryCap = 1u << 16;  // CAS retries per union
 constexpr uint32_t kLookbackSpinCap = 1u << 20; // waits per look-back window (~1 s)
 
 // ---------------------------------------------------------------- device control block
 // Small per-context device structure, zeroed at the start of each solve.
+constexpr uint32_t kMaxBarriers = 3 * PHEM_MAX_ROUNDS + 8;  // grid barriers of one MSF solve
+constexpr uint32_t kMaxPhases = kMaxBarriers + 8;
 struct Ctl {
     uint32_t err;
-    uint32_t round;                                  // device-side round counter
-    uint32_t go;                                     // 1 while another round is needed
-    uint32_t phase;                                  // 0: light edges, 1: heavy edges
-    uint32_t src;                                    // input of this round's edge pass (kSrc*)
-    uint32_t cand_all;                               // this round's candidates are all n vertices
+    uint32_t round;                                  // Boruvka rounds run
     uint32_t light_rounds;                           // rounds spent in the light phase
-    uint32_t pad0;
+    uint32_t ticket;                                 // tile tickets (R-MAT generator)
     unsigned long long threshold;                    // light edge <=> key < threshold
     unsigned long long m_r[PHEM_MAX_ROUNDS + 1];     // live edges entering round r (exact)
-    unsigned long long wl_len[PHEM_MAX_ROUNDS + 1];  // records written by round r's edge pass,
-                                                     // including dead padding at chunk tails
     unsigned long long n_r[PHEM_MAX_ROUNDS + 1];     // components with a live edge in round r
-    uint32_t roots[PHEM_MAX_ROUNDS + 2];             // |candidate roots| entering round r
-    uint32_t ticket[PHEM_MAX_ROUNDS + 2];            // tile tickets of the round's edge pass
-    uint32_t out_ticket;                             // tile tickets of the output gather
-    uint32_t pad1;
     unsigned long long msf_count;
     unsigned long long msf_total;
     unsigned long long misc[8];
+    // from here on only the device (and profiling) looks
+    unsigned long long bar[kMaxBarriers];            // one word per grid barrier of the MSF solve
+    unsigned long long stamp[kMaxPhases];            // profiling: end time of each phase (ns)
+    uint32_t phase_of[kMaxPhases];                   // ... and the phase's name (KernelId)
+    uint32_t stamps;
+    uint32_t pad0;
 };
 
 // Input of an edge pass.
 enum : uint32_t {
     kSrcLight = 0,  // the caller's edges, keeping key < threshold; endpoints are their own roots
-    kSrcList = 1,   // the previous round's survivor records
+    kSrcList = 1,   // the previous round's survivor records, per warp
     kSrcHeavy = 2,  // the caller's edges, keeping key >= threshold; endpoints relabelled by parent[]
 };
 
@@ -83,30 +79,6 @@ __device__ __forceinline__ void st_relaxed_u64(uint64_t *p, uint64_t v)
 __device__ __forceinline__ void set_err(uint32_t *err, uint32_t bit) { atomicOr(err, bit); }
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
-
-// ---------------------------------------------------------------- warp-aggregated minimum
-// Lanes with valid == true offer `key` to slot best[target]; lanes sharing a
-// target are reduced first (__match_any_sync groups them; the 64-bit key is
-// reduced as (high word, then low word among lanes holding the minimum high
-// word) with __reduce_min_sync), then one guarded atomicMin per group.  Every
-// lane of the warp must call this with the warp converged.
-__device__ __forceinline__ void warp_min_to(unsigned long long *best, uint32_t target, uint64_t key,
-                                            bool valid)
-{
-    const unsigned active = __ballot_sync(0xffffffffu, valid);
-    if (!valid)
-        return;
-    const unsigned peers = __match_any_sync(active, target);
-    const uint32_t hi = (uint32_t)(key >> 32), lo = (uint32_t)key;
-    const uint32_t mhi = __reduce_min_sync(peers, hi);
-    const uint32_t mlo = __reduce_min_sync(peers, hi == mhi ? lo : 0xffffffffu);
-    if ((int)lane_id() == __ffs(peers) - 1) {
-        const unsigned long long k = ((unsigned long long)mhi << 32) | mlo;
-        if (k < __ldcg(best + target))
-            atomicMin(best + target, k);
-    }
-}
-
 
 // ---------------------------------------------------------------- block scan
 // Exclusive scan of one uint32 per thread over a kBlock-thread block.

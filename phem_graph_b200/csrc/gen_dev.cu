@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(kGenThreads) rmat_range_kernel(RmatParams p, u
     const uint64_t ntiles = (count + kGenTile - 1) / kGenTile;
     for (;;) {
         if (threadIdx.x == 0)
-            s_tile = atomicAdd(&ctl->ticket[0], 1u);
+            s_tile = atomicAdd(&ctl->ticket, 1u);
         __syncthreads();
         const uint32_t t = s_tile;
         if (t >= ntiles)

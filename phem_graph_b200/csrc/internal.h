@@ -14,7 +14,8 @@
 namespace phem {
 // Kernels the library launches; the profile reports them by these names.
 enum KernelId : int {
-    kKInit = 0, kKSelect, kKEdgePass, kKHook, kKCompress, kKAdvance, kKGather,
+    kKSolve = 0,  // the MSF solve; the next six are its phases (device timestamps, no launches)
+    kKInit, kKSelect, kKEdgePass, kKHook, kKCompress, kKGather,
     kKCcInit, kKCcUnite, kKCcMerge, kKCcLabel, kKMinid, kKCcCount, kKCsrCoo, kKBatch,
     kKernelCount
 };
@@ -56,22 +57,15 @@ struct phem_context {
     uint64_t epoch = 1;                // look-back epoch counter
     uint32_t timeout_ms = 0;
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
-    int edge_pass_blocks = 0;          // persistent grid sizes, from the occupancy API
     uint32_t kernels_ready = 0;        // bit k: launch attributes of edge kind k are set
-    int gather_blocks = 0;
-    int tune_edge_ctas = 4;              // MSF edge pass: CTAs (of 8 independent warps) per SM, 1 to 4
-    int tune_graph = 1;                  // MSF rounds as a CUDA graph with a device-driven while-node
-    cudaGraphExec_t msf_exec[2] = {nullptr, nullptr};  // cached round-loop graphs, per edge kind
-    uint64_t msf_key[2][40] = {};        // what each was built for
-    uint64_t msf_seen[2][40] = {};       // the last solve's key (a graph is built when it repeats)
-    bool msf_graph_pending = false;      // a graph solve's launches are still to be counted
-    bool msf_graph_select = false;       // ... and it had a threshold select
+    int tune_edge_ctas = 4;              // MSF solve: groups of 8 independent warps per SM, 1 to 4
+    int tune_graph = 1;                  // kept for callers that set them: the rounds always
+    int tune_first_batch = 12;           // run inside the one solve launch
+    int tune_next_batch = 4;
     // tuning knobs (phem_context_set_tuning)
     double tune_light_per_vertex = 0.5;  // light edges per vertex in the MSF filter (0: no filter)
     double tune_canonical_light = 1.5;   // the same for the canonical CC forest (edges by index)
     double tune_filter_min_ratio = 2.0;  // filter only when m >= ratio * light edges
-    int tune_first_batch = 12;           // Boruvka rounds queued before the first host check
-    int tune_next_batch = 4;             // rounds queued per later check
     int tune_batch_block = 1024;         // batched kernel: threads per CTA
     int tune_batch_items = 4;            // batched kernel: records per thread per step
     double tune_batch_compact = 1.0;     // batched kernel: compaction threshold
@@ -151,6 +145,8 @@ struct KernelScope {
 };
 // Folds finished event pairs into the per-kernel totals (call after a sync).
 void resolve_timings(phem_context *ctx);
+// Adds one timed phase of a kernel (device timestamps).
+void log_phase(phem_context *ctx, int kernel, float ms);
 
 // ---- call helpers shared by the entry points ----
 
@@ -251,31 +247,28 @@ struct MsfPlan {
     uint64_t m;
     uint32_t n;
     uint32_t *parent;        // n
-    unsigned long long *best;// n
-    uint32_t *cand;          // n: the round's choosers (hook -> compress)
-    uint32_t *samples;       // 8192: the threshold select's sampled weights
+    unsigned long long *best;// two arrays of best_stride words, by round parity
+    uint64_t best_stride;    // >= n
+    uint32_t *samples;       // the threshold select's sampled weights
     uint32_t *bitmap;        // ceil(m / 32)
     uint32_t *chunk_cnt;     // MSF edges per 1024 edge ids, then their offsets (gather)
-    uint4 *wl[2];            // m each
-    uint64_t *status;        // look-back status (context-owned), >= tiles
-    uint64_t epoch_base;
+    uint32_t *cta_tot;       // forest edges per CTA's range (gather)
+    uint32_t *giant;         // one bit per vertex
+    uint4 *list;             // survivor segments, one per warp
+    uint32_t *hooked;        // hooked-root segments, one per warp
     uint64_t *forest;        // kKindPacked only: forest slot per hooked root (may be null)
+    phem_edge *out;          // kKindMsf with gather: the ordered MSF records (may be null)
+    int gather;              // kKindMsf: rank and write the MSF records, count and total
 };
 
 size_t msf_workspace_bytes(uint64_t m, uint32_t n, int sm_count);
-phem_status msf_plan(phem_context *ctx, int kind, const void *d_e0, uint64_t m, uint32_t n, size_t extra_bytes,
-                     MsfPlan *plan, size_t *extra_off);
-// Queues the whole Boruvka solve; returns after the rounds are done and
-// checked (the stream form checks the round flag between batches).  With
-// `deferred` the graph form returns once the rounds are queued, and the
-// caller queues more work before msf_finish waits and checks.  After the
-// rounds the bitmap marks the MSF.
-phem_status msf_run(phem_context *ctx, int kind, MsfPlan &plan, uint32_t *rounds_out, bool deferred = false);
-// Waits for the queued work and checks the rounds (copies the control block
+phem_status msf_plan(phem_context *ctx, const void *d_e0, uint64_t m, uint32_t n, size_t extra_bytes, MsfPlan *plan,
+                     size_t *extra_off);
+// Queues the whole solve (one launch); msf_finish waits and checks.
+phem_status msf_run(phem_context *ctx, int kind, MsfPlan &plan);
+// Waits for the queued work and checks it (copies the control block's results
 // to ctx->h_ctl).
-phem_status msf_finish(phem_context *ctx, uint32_t *rounds_out);
-// Queues the ordered gather of MSF edges (kKindMsf): out[0..count) + count/total into ctl.
-phem_status msf_gather(phem_context *ctx, MsfPlan &plan, phem_edge *d_out);
+phem_status msf_finish(phem_context *ctx, uint32_t *rounds_out, const char *what);
 
 // ---- CC engine (cc.cu) ----
 phem_status cc_launch_init(phem_context *ctx, int32_t n, int32_t *parent, int32_t *label, uint64_t *forest);

@@ -324,3 +324,30 @@ def test_graph_and_stream_round_loops(ctx, graph):
         np.testing.assert_array_equal(P.api.forest_set(rc.forest), oracle.forest_set(forest))
     finally:
         ctx.set_tuning("msf.graph", old)
+
+
+@pytest.mark.parametrize("m", [1, 31, 128, 129, 191, 193, 4095, 16383, 16384, 16385, 16513, 32769, 1048573])
+def test_one_launch_solve_sizes(ctx, m):
+    """Sizes around the solve kernel's tiles (128 records, 192 pairs), the
+    step from one CTA to a grid, and remainders, for weighted and packed
+    edges; bit-exact against Kruskal."""
+    n = max(2, m // 6)
+    pairs = gen.er(n, m + m // 64 + 8, seed=m)[:m]
+    E = gen.msf_edges(pairs, gen.weights(len(pairs), m, bits=10))
+    ids, cnt, tot = expect(E, n)
+    assert_msf(ctx.msf_solve(E, n), E, ids, cnt, tot)
+    labels, forest = oracle.cc_solve(pairs, n)
+    rc = ctx.cc_solve(pairs, n, canonical=True)
+    np.testing.assert_array_equal(rc.labels, labels)
+    np.testing.assert_array_equal(P.api.forest_set(rc.forest), oracle.forest_set(forest))
+
+
+@pytest.mark.parametrize("n", [3, 1000, 40000])
+def test_long_hook_chains(ctx, n):
+    """A path with ascending weights hooks into one chain of n vertices in
+    round 0 (the compress has to walk it)."""
+    u = np.arange(n - 1, dtype=np.uint32)
+    E = np.ascontiguousarray(np.stack([u, u + 1, u + 1], axis=1))
+    r = ctx.msf_solve(E, n)
+    assert (r.count, r.total) == (n - 1, n * (n - 1) // 2)
+    np.testing.assert_array_equal(r.edges, E)
