@@ -9,9 +9,11 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <cstdlib>
 #include <thread>
 
 #include "internal.h"
+#include "tiny.h"
 
 namespace phem {
 
@@ -326,6 +328,8 @@ void phem_context_destroy(phem_context *ctx)
         cudaFree(ctx->ctl);
     if (ctx->h_ctl)
         cudaFreeHost(ctx->h_ctl);
+    if (ctx->tiny_host)
+        cudaFreeHost(ctx->tiny_host);
     if (ctx->ev_start)
         cudaEventDestroy(ctx->ev_start);
     if (ctx->ev_stop)
@@ -586,6 +590,46 @@ static phem_status cc_unite_overlapped(phem_context *ctx, const uint64_t *h_edge
     return st;
 }
 
+// phem_cc_solve for a graph that one CTA solves.
+static phem_status cc_solve_tiny(phem_context *ctx, const uint64_t *edges, int64_t m, int32_t n, int32_t *labels,
+                                 uint64_t *forest, bool canonical, phem_cc_stats *stats)
+{
+    const size_t eb = (size_t)m * sizeof(uint64_t), lb = (size_t)n * sizeof(int32_t),
+                 fb = (size_t)n * sizeof(uint64_t);
+    const size_t o_lab = align256(eb), o_for = o_lab + align256(lb);
+    PHEM_TRY(ws_reserve(ctx, o_for + align256(fb)));
+    const void *in = nullptr;
+    PHEM_TRY(tiny_input(ctx, edges, eb, ctx->ws, &in));
+    Staged sl, sf;
+    stage_out(ctx, labels, lb, o_lab, &sl);
+    stage_out(ctx, forest, fb, o_for, &sf);
+    const uint64_t *e = static_cast<const uint64_t *>(in);
+    cudaEventRecord(ctx->ev_start, ctx->stream);
+    if (canonical) {
+        const uint64_t k = canonical_light(ctx, m, n);
+        PHEM_TRY(tiny_canonical(ctx, e, (uint32_t)m, (uint32_t)n, k ? k : kKeyNone, static_cast<int32_t *>(sl.dev),
+                                static_cast<uint64_t *>(sf.dev)));
+    } else {
+        PHEM_TRY(tiny_cc(ctx, e, (uint32_t)m, (uint32_t)n, static_cast<int32_t *>(sl.dev),
+                         static_cast<uint64_t *>(sf.dev)));
+    }
+    cudaEventRecord(ctx->ev_stop, ctx->stream);
+    PHEM_TRY(copy_back(ctx, sl, lb));
+    PHEM_TRY(copy_back(ctx, sf, fb));
+    PHEM_TRY(stream_wait(ctx));
+    const Ctl &h = *ctx->h_ctl;
+    PHEM_TRY(ctl_status(h.err, "cc_solve"));
+    if (stats) {
+        stats->components = (uint32_t)h.misc[0];
+        stats->forest_edges = h.misc[1];
+        stats->rounds = h.round;
+        stats->device_ms = 0.f;
+        if (cudaEventElapsedTime(&stats->device_ms, ctx->ev_start, ctx->ev_stop) != cudaSuccess)
+            stats->device_ms = 0.f;
+    }
+    return PHEM_OK;
+}
+
 phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, int32_t n, int32_t *labels,
                           uint64_t *forest, uint32_t flags, phem_cc_stats *stats)
 {
@@ -600,6 +644,8 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
         return PHEM_ERR_INVALID;
     }
     DeviceGuard g(ctx->device);
+    if (canonical ? tiny_msf_fits((uint64_t)m, (uint64_t)n) : tiny_cc_fits(m, n))
+        return cc_solve_tiny(ctx, edges, m, n, labels, forest, canonical, stats);
     const size_t eb = (size_t)m * sizeof(uint64_t), lb = (size_t)n * sizeof(int32_t),
                  fb = (size_t)n * sizeof(uint64_t);
     // extra area: staged edges | labels | forest | parent (default path)
@@ -917,6 +963,56 @@ phem_status phem_cc_merge(phem_context *ctx, const uint64_t *d_forest_a, const u
 
 // ------------------------------------------------------------------ MSF
 
+// The finished solve's figures out of the control block's mirror.
+static void msf_results(phem_context *ctx, uint64_t *count, uint64_t *total, phem_msf_stats *stats)
+{
+    const Ctl &h = *ctx->h_ctl;
+    if (count)
+        *count = h.msf_count;
+    if (total)
+        *total = h.msf_total;
+    if (!stats)
+        return;
+    std::memset(stats, 0, sizeof(*stats));
+    stats->rounds = h.round;
+    for (uint32_t r = 0; r < h.round && r < PHEM_MAX_ROUNDS; r++) {
+        stats->m_r[r] = h.m_r[r];
+        stats->n_r[r] = h.n_r[r];
+    }
+    stats->light_rounds = h.light_rounds;
+    stats->threshold = h.threshold;
+    stats->msf_edges = h.msf_count;
+    stats->total_weight = h.msf_total;
+    if (cudaEventElapsedTime(&stats->device_ms, ctx->ev_start, ctx->ev_stop) != cudaSuccess)
+        stats->device_ms = 0.f;
+}
+
+// A graph that one CTA solves.
+static phem_status msf_tiny(phem_context *ctx, const phem_edge *edges, uint64_t m, uint32_t n, phem_edge *msf,
+                            uint64_t *count, uint64_t *total, phem_msf_stats *stats, uint64_t *d_count_total)
+{
+    const size_t eb = (size_t)m * sizeof(phem_edge);
+    PHEM_TRY(ws_reserve(ctx, align256(eb)));
+    const void *in = nullptr;
+    PHEM_TRY(tiny_input(ctx, edges, eb, ctx->ws, &in));
+    phem_edge *out = msf;
+    char *host = nullptr;
+    if (msf && !is_device_ptr(msf)) {
+        PHEM_TRY(tiny_host(ctx, &host));
+        out = reinterpret_cast<phem_edge *>(host + kTinyHostOut);
+    }
+    cudaEventRecord(ctx->ev_start, ctx->stream);
+    PHEM_TRY(tiny_msf(ctx, static_cast<const phem_edge *>(in), (uint32_t)m, n, out, d_count_total));
+    cudaEventRecord(ctx->ev_stop, ctx->stream);
+    PHEM_TRY(stream_wait(ctx));
+    if(getenv("PHEM_ST")) {for(uint32_t q=0;q<ctx->h_ctl->stamps;q++) printf("%.2f ",(double)ctx->h_ctl->stamp[q]/1900.); printf("\n");fflush(stdout);}
+    PHEM_TRY(ctl_status(ctx->h_ctl->err, "msf"));
+    if (host)
+        std::memcpy(msf, out, ctx->h_ctl->msf_count * sizeof(phem_edge));
+    msf_results(ctx, count, total, stats);
+    return PHEM_OK;
+}
+
 static phem_status msf_common(phem_context *ctx, const phem_edge *edges, uint64_t m, uint32_t n, phem_edge *msf,
                               uint64_t *count, uint64_t *total, phem_msf_stats *stats, uint64_t *d_count_total)
 {
@@ -924,6 +1020,8 @@ static phem_status msf_common(phem_context *ctx, const phem_edge *edges, uint64_
         set_error("msf: need 0 < n < 2^32 - 1, m <= 2^32 - 2^24 and an edge array");
         return PHEM_ERR_INVALID;
     }
+    if (tiny_msf_fits(m, n))
+        return msf_tiny(ctx, edges, m, n, msf, count, total, stats, d_count_total);
     const bool aligned_dev = is_device_ptr(edges) && (((uintptr_t)edges & 15) == 0);
     const size_t eb = (size_t)m * sizeof(phem_edge), ob = (size_t)n * sizeof(phem_edge);
     const size_t o_edges = 0, o_out = aligned_dev ? 0 : align256(eb);  // edges read in place: no staging area
@@ -950,9 +1048,6 @@ static phem_status msf_common(phem_context *ctx, const phem_edge *edges, uint64_
         PHEM_CUDA_TRY(cudaMemcpyAsync(d_count_total, &ctx->ctl->msf_count, 2 * sizeof(uint64_t),
                                       cudaMemcpyDeviceToDevice, ctx->stream));
     PHEM_TRY(msf_finish(ctx, &rounds, "msf"));
-    float ms = 0.f;
-    if (cudaEventElapsedTime(&ms, ctx->ev_start, ctx->ev_stop) != cudaSuccess)
-        ms = 0.f;
     const Ctl &h = *ctx->h_ctl;
     if (h.msf_count > (uint64_t)n - 1 + (n == 0)) {
         set_error("msf: %llu forest edges for %u vertices", (unsigned long long)h.msf_count, n);
@@ -960,23 +1055,7 @@ static phem_status msf_common(phem_context *ctx, const phem_edge *edges, uint64_
     }
     if (so.host && h.msf_count)
         PHEM_CUDA_TRY(cudaMemcpy(so.host, so.dev, h.msf_count * sizeof(phem_edge), cudaMemcpyDeviceToHost));
-    if (count)
-        *count = h.msf_count;
-    if (total)
-        *total = h.msf_total;
-    if (stats) {
-        std::memset(stats, 0, sizeof(*stats));
-        stats->rounds = rounds;
-        for (uint32_t r = 0; r < rounds && r < PHEM_MAX_ROUNDS; r++) {
-            stats->m_r[r] = h.m_r[r];
-            stats->n_r[r] = h.n_r[r];
-        }
-        stats->light_rounds = h.light_rounds;
-        stats->threshold = h.threshold;
-        stats->msf_edges = h.msf_count;
-        stats->total_weight = h.msf_total;
-        stats->device_ms = ms;
-    }
+    msf_results(ctx, count, total, stats);
     return PHEM_OK;
 }
 

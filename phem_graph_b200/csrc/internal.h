@@ -54,6 +54,8 @@ struct phem_context {
     size_t status_words = 0;           // (zeroed when grown; epochs keep old words from matching)
     phem::Ctl *ctl = nullptr;          // device control block
     phem::Ctl *h_ctl = nullptr;        // pinned host mirror of the control block
+    void *tiny_host = nullptr;         // pinned staging of small host solves (tiny.cu), made on first use
+    uint32_t tiny_ready = 0;           // bit k: launch attributes of small-solve kernel k are set
     uint64_t epoch = 1;                // look-back epoch counter
     uint32_t timeout_ms = 0;
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
@@ -261,6 +263,8 @@ struct MsfPlan {
     int gather;              // kKindMsf: rank and write the MSF records, count and total
 };
 
+// The canonical forest's light edges (the first ones by index; 0: no split).
+uint64_t canonical_light(phem_context *ctx, uint64_t m, uint64_t n);
 size_t msf_workspace_bytes(uint64_t m, uint32_t n, int sm_count);
 phem_status msf_plan(phem_context *ctx, const void *d_e0, uint64_t m, uint32_t n, size_t extra_bytes, MsfPlan *plan,
                      size_t *extra_off);

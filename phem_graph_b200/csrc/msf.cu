@@ -1109,6 +1109,14 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(const __grid_co
     }
 }
 
+// Light/heavy split: about lpv * n light edges, and only when the input is at
+// least filter_min_ratio times that large (0: no split).
+uint64_t light_edges(phem_context *ctx, double lpv, uint64_t m, uint64_t n)
+{
+    const uint64_t k = (uint64_t)(lpv * (double)n);
+    return lpv > 0 && (double)m >= ctx->tune_filter_min_ratio * (double)k ? k : 0;
+}
+
 // Sampled weights: enough that the light count is within a few per cent of
 // its aim where it matters (a small input's select is part of its latency).
 uint32_t sample_count(uint64_t m) { return m >= (1u << 22) ? kMaxSample : 2048; }
@@ -1170,16 +1178,13 @@ phem_status run_impl(phem_context *ctx, MsfPlan &plan)
     a.gather = plan.gather;
     a.ctl = ctx->ctl;
     a.timing = ctx->profiling;
-    // light/heavy split: about light_per_vertex * n light edges, and only when
-    // the input is at least filter_min_ratio times that large
-    // the canonical forest's light edges are the first ones by index, which
-    // start forming the large components only at about two per vertex
-    const double lpv = KIND == kKindPacked ? ctx->tune_canonical_light : ctx->tune_light_per_vertex;
-    const uint64_t k = (uint64_t)(lpv * (double)plan.n);
-    const bool filter = lpv > 0 && k > 0 && (double)plan.m >= ctx->tune_filter_min_ratio * (double)k;
-    a.light_k = filter ? k : plan.m;
-    a.threshold = filter && KIND == kKindPacked ? k : kKeyNone;  // packed: the first k edges are light
-    a.nsamp = filter && KIND == kKindMsf ? sample_count(plan.m) : 0;
+    // packed edges: the first k by index are light; the canonical forest's
+    // slots follow from the rounds, so this rule is the same at every size
+    const uint64_t k = KIND == kKindPacked ? canonical_light(ctx, plan.m, plan.n)
+                                           : light_edges(ctx, ctx->tune_light_per_vertex, plan.m, plan.n);
+    a.light_k = k ? k : plan.m;
+    a.threshold = k && KIND == kKindPacked ? k : kKeyNone;
+    a.nsamp = k && KIND == kKindMsf ? sample_count(plan.m) : 0;
     const int threads = 256 * ctx->tune_edge_ctas;
     const uint32_t blocks = solve_blocks(plan.m, ctx->sm_count);
     a.seg = seg_records(plan.m, blocks * (uint32_t)(threads / 32), KIND == kKindMsf ? 12 : 8);
@@ -1195,6 +1200,11 @@ phem_status run_impl(phem_context *ctx, MsfPlan &plan)
 }
 
 }  // namespace
+
+uint64_t canonical_light(phem_context *ctx, uint64_t m, uint64_t n)
+{
+    return light_edges(ctx, ctx->tune_canonical_light, m, n);
+}
 
 // Records all segments may need: every edge plus one tile per warp.
 uint64_t list_capacity(uint64_t m, int sm_count)

@@ -351,3 +351,32 @@ def test_long_hook_chains(ctx, n):
     r = ctx.msf_solve(E, n)
     assert (r.count, r.total) == (n - 1, n * (n - 1) // 2)
     np.testing.assert_array_equal(r.edges, E)
+
+
+@pytest.mark.parametrize("n,m", [(2, 1), (37, 4095), (300, 4096), (1021, 4097), (2000, 8192), (2000, 8193),
+                                 (16384, 16384), (16383, 3000), (16385, 9000), (5000, 16385)])
+def test_one_cta_solve_sizes(ctx, n, m):
+    """Small graphs solved by one CTA: sizes around the records-per-thread
+    steps and the limits, weight ties, host and (12-byte offset) device
+    inputs, both kinds of CC forest."""
+    import torch
+    pairs = gen.er(n, 2 * m + 8, seed=m)[:m]
+    assert len(pairs) == m
+    E = gen.msf_edges(pairs, gen.weights(m, m, bits=6))
+    ids, cnt, tot = expect(E, n)
+    assert_msf(ctx.msf_solve(E, n), E, ids, cnt, tot)
+    d = torch.from_numpy(np.concatenate([E[:1], E]).view(np.int32)).cuda()[1:]
+    out = torch.zeros((n, 3), dtype=torch.int32, device="cuda")
+    ct = torch.zeros(2, dtype=torch.int64, device="cuda")
+    r = ctx.msf_solve_device(d, m, n, out, ct)
+    assert (r.count, r.total) == (cnt, tot) and ct.tolist() == [cnt, tot]
+    np.testing.assert_array_equal(out.cpu().numpy().view(np.uint32)[:cnt], E[ids])
+    labels, forest = oracle.cc_solve(pairs, n)
+    rc = ctx.cc_solve(pairs, n, canonical=True)
+    np.testing.assert_array_equal(rc.labels, labels)
+    np.testing.assert_array_equal(P.api.forest_set(rc.forest), oracle.forest_set(forest))
+    rd = ctx.cc_solve(pairs, n)
+    np.testing.assert_array_equal(rd.labels, labels)
+    f = P.api.forest_set(rd.forest)
+    assert rd.components == rc.components == n - len(f) == n - rd.forest_edges
+    np.testing.assert_array_equal(oracle.cc_solve(f, n)[0], labels)
