@@ -115,7 +115,8 @@ phem_status phem_context_launch_log(phem_context *ctx, phem_launch_record *out, 
 
 /* Tuning knobs (defaults suit B200; the autotuner may change them):
  *   "msf.light_per_vertex"  light edges per vertex taken by the MSF filter
- *                           before the heavy pass; 0 disables the filter   [0.5]
+ *                           before the heavy pass (twice as many when the
+ *                           sampled degrees are even); 0 disables it       [0.5]
  *   "msf.filter_min_ratio"  filter only when m >= ratio * light edges      [2.0]
  *   "msf.edge_ctas_per_sm"  groups of 8 warps per SM in the solve, 1 to 4 [4]
  *   "msf.first_batch", "msf.next_batch", "msf.graph"  accepted and without

@@ -65,7 +65,7 @@ struct SolveArgs {
     uint32_t *parent;
     unsigned long long *best;      // two arrays of best_stride words: minimum key offered, by round parity
     uint64_t best_stride;
-    uint32_t *samples;             // sampled weights of the threshold select
+    uint32_t *samples;             // the threshold select's sample: weights, then one endpoint each
     uint32_t nsamp;                // 0: no select
     uint32_t *bitmap;              // MSF membership, one bit per edge id
     uint32_t *chunk_cnt;           // MSF edges per 1024 edge ids, then their offsets within a CTA's range
@@ -78,7 +78,7 @@ struct SolveArgs {
     phem_edge *out;
     Ctl *ctl;
     unsigned long long threshold;  // when nothing is selected
-    uint64_t light_k;              // light edges the threshold aims at
+    uint64_t light_k, light_k2;    // light edges the threshold aims at: skewed degrees, even ones
     int gather;                    // write the ordered MSF records (kKindMsf)
     int timing;                    // record phase timestamps
 };
@@ -86,6 +86,7 @@ struct SolveArgs {
 constexpr int kSolveThreads = 1024;  // most threads per CTA (one CTA per SM); 64 registers each
 constexpr int kSolveWarps = kSolveThreads / 32;
 constexpr uint32_t kMaxSample = 8192;
+constexpr uint32_t kSeenWords = 8192;  // 2^18 bits
 constexpr uint32_t kMaxGrid = 1024;
 
 // Count words for the chunks of 1024 edge ids (32 bitmap words).
@@ -154,10 +155,10 @@ struct SolveSmem {
     uint32_t fatal;             // a bounded wait of this CTA gave up
     uint32_t scan[kSolveWarps + 1];
     uint32_t pref[kMaxGrid];    // forest edges of the CTA ranges before each (gather)
-    uint32_t sel_prefix, sel_rank, sel_or;
+    uint32_t sel_prefix, sel_rank, sel_or, sel_dup;
 };
-static_assert(sizeof(EpWarp) * kSolveWarps >= (kMaxSample + 2048) * sizeof(uint32_t),
-              "the select's samples and histogram fit in the warps' space");
+static_assert(sizeof(EpWarp) * kSolveWarps >= (kMaxSample + kSeenWords) * sizeof(uint32_t),
+              "the select's samples, set and histogram fit in the warps' space");
 
 // Grid barrier with a sum: adds the CTAs' `acc`, returns false when the solve
 // has to stop (a bounded wait gave up somewhere; the status bit says so).  One
@@ -275,29 +276,48 @@ __device__ __forceinline__ uint64_t sample_pos(uint32_t i, uint32_t count, uint6
     return hi > lo ? lo + mix64(0x5EED0000ull + i) % (hi - lo) : lo;
 }
 
-// The sample's rank-th smallest weight (rank = light_k scaled to the sample):
-// a three-digit radix select in shared memory, run by every CTA on the same
-// sample instead of by one CTA and a further barrier.
+// The sample's rank-th smallest weight (rank = the light edges aimed at, scaled
+// to the sample): a three-digit radix select in shared memory, run by every
+// CTA on the same sample instead of by one CTA and a further barrier.
+//
+// How many light edges pay depends on the degrees: the light phase has to
+// build the component that filters the heavy edges, which takes well over n/2
+// edges when all degrees are alike and far fewer when hubs collect them.  The
+// sample tells the two apart: endpoints that repeat (in a hashed set of 2^18)
+// several times as often as uniform ones would mean hubs.  us per solve at
+// 0.5 / 1 light edges per vertex: R-MAT 22 1065 / 1102; uniform n = 2^20, m =
+// 2^23 844 / 542, n = 131,101, m = 2^20 302 / 232; geometric n = 262,147
+// 315 / 304.
 __device__ __forceinline__ unsigned long long select_threshold(const SolveArgs &a, SolveSmem &s)
 {
     uint32_t *samp = reinterpret_cast<uint32_t *>(s.warp);
     uint32_t *hist = samp + kMaxSample;
     const uint32_t S = a.nsamp, tid = threadIdx.x, lane = lane_id();
-    if (tid == 0) {
-        s.sel_prefix = 0;
-        s.sel_rank = (uint32_t)(a.light_k * S / a.m);
-        s.sel_or = 0;
-    }
+    if (tid == 0)
+        s.sel_prefix = s.sel_or = s.sel_dup = 0;
+    uint32_t *seen = hist;  // 2^18 bits, before the histograms
+    for (uint32_t i = tid; i < kSeenWords / 4; i += blockDim.x)
+        reinterpret_cast<uint4 *>(seen)[i] = make_uint4(0, 0, 0, 0);
     __syncthreads();
-    uint32_t orv = 0;
+    uint32_t orv = 0, dup = 0;
     for (uint32_t i = tid; i < S; i += blockDim.x) {
-        const uint32_t x = __ldcg(a.samples + i);
+        const uint32_t x = __ldcg(a.samples + i), v = __ldcg(a.samples + S + i);
         samp[i] = x;
         orv |= x;
+        const uint32_t h = (v * 0x9E3779B1u) >> 14, bit = 1u << (h & 31);
+        dup += (atomicOr(&seen[h >> 5], bit) & bit) != 0;
     }
     orv = __reduce_or_sync(0xffffffffu, orv);
-    if (lane == 0)
+    dup = __reduce_add_sync(0xffffffffu, dup);
+    if (lane == 0) {
         atomicOr(&s.sel_or, orv);
+        atomicAdd(&s.sel_dup, dup);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        const float even = 0.5f * (float)S * (float)S * (1.f / (32.f * kSeenWords) + 1.f / (float)a.n);
+        s.sel_rank = (uint32_t)(((float)s.sel_dup > 4.f * even + 32.f ? a.light_k : a.light_k2) * S / a.m);
+    }
 #pragma unroll
     for (int d = 0; d < 3; d++) {
         const int sh = d == 0 ? 21 : (d == 1 ? 10 : 0), nb = d == 2 ? 10 : 11, hsh = sh + nb;
@@ -1000,8 +1020,11 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(const __grid_co
     // init
     {
         const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + tid, T = (uint64_t)gridDim.x * blockDim.x;
-        for (uint64_t i = g; i < a.nsamp; i += T)
-            a.samples[i] = __ldg(static_cast<const uint32_t *>(a.e0) + sample_pos((uint32_t)i, a.nsamp, a.m) * 3 + 2);
+        for (uint64_t i = g; i < a.nsamp; i += T) {
+            const uint32_t *e = static_cast<const uint32_t *>(a.e0) + sample_pos((uint32_t)i, a.nsamp, a.m) * 3;
+            a.samples[i] = __ldg(e + 2);
+            a.samples[a.nsamp + i] = __ldg(e + (i & 1));
+        }
         for (uint64_t x = g; x < a.n; x += T) {
             a.parent[x] = (uint32_t)x;
             a.best[x] = kKeyNone;
@@ -1117,6 +1140,11 @@ uint64_t light_edges(phem_context *ctx, double lpv, uint64_t m, uint64_t n)
     return lpv > 0 && (double)m >= ctx->tune_filter_min_ratio * (double)k ? k : 0;
 }
 
+// Below this many edges the weighted solve runs unfiltered: a light phase's
+// rounds cost their barriers whatever they find.  us per solve without / with
+// the filter: m = 100,003 137 / 152, m = 200,000 163 / 188, m = 2^20 276 / 238.
+constexpr uint64_t kFilterMinEdges = 240000;
+
 // Sampled weights: enough that the light count is within a few per cent of
 // its aim where it matters (a small input's select is part of its latency).
 uint32_t sample_count(uint64_t m) { return m >= (1u << 22) ? kMaxSample : 2048; }
@@ -1135,7 +1163,7 @@ phem_status setup_kernel(phem_context *ctx)
                                        (int)sizeof(SolveSmem)));
     int per_sm = 0;
     PHEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, solve_kernel<KIND>,
-                                                                256 * ctx->tune_edge_ctas, sizeof(SolveSmem)));
+                                                                kSolveThreads, sizeof(SolveSmem)));
     if (per_sm < 1) {
         set_error("msf: the solve kernel does not fit on an SM");
         return PHEM_ERR_UNSUPPORTED;
@@ -1143,12 +1171,25 @@ phem_status setup_kernel(phem_context *ctx)
     return PHEM_OK;
 }
 
-// CTAs of a solve: one per SM, fewer for small inputs.
-uint32_t solve_blocks(uint64_t m, int sm_count)
+// CTAs and threads of a solve.  A warp gets at least one tile; a small input
+// runs more CTAs of fewer warps (more SMs' load queues, and a block barrier
+// among fewer warps), a large one needs the warps.  us per solve with 256 /
+// 512 / 1024 threads: m = 100,003 137 / 138 / 161; m = 200,000 183 / 163 /
+// 198; m = 2^20 250 / 238 / 250; m = 4,000,000 442 / 373 / 361.
+struct SolveGrid {
+    uint32_t blocks;
+    int threads;
+};
+SolveGrid solve_grid(uint64_t m, uint32_t rec_bytes, int sm_count, int max_groups)
 {
-    const uint64_t tiles = (m + 127) / 128;
-    const uint64_t want = tiles <= 4 * kSolveWarps ? 1 : (tiles + 2 * kSolveWarps - 1) / (2 * kSolveWarps);
-    return (uint32_t)std::min<uint64_t>(std::min<uint64_t>(want, (uint64_t)sm_count), kMaxGrid);
+    const uint64_t tile = kEpStageBytes / rec_bytes, tiles = (m + tile - 1) / tile;
+    const int groups = tiles <= 8 * (uint64_t)sm_count ? 1 : (tiles <= 64 * (uint64_t)sm_count ? 2 : 4);
+    SolveGrid g;
+    g.threads = 256 * std::min(groups, max_groups);
+    const uint64_t warps = (uint64_t)g.threads / 32;
+    g.blocks = (uint32_t)std::max<uint64_t>(
+        1, std::min({(tiles + warps - 1) / warps, (uint64_t)sm_count, (uint64_t)kMaxGrid}));
+    return g;
 }
 
 template <int KIND>
@@ -1181,20 +1222,25 @@ phem_status run_impl(phem_context *ctx, MsfPlan &plan)
     // packed edges: the first k by index are light; the canonical forest's
     // slots follow from the rounds, so this rule is the same at every size
     const uint64_t k = KIND == kKindPacked ? canonical_light(ctx, plan.m, plan.n)
-                                           : light_edges(ctx, ctx->tune_light_per_vertex, plan.m, plan.n);
+                       : plan.m < kFilterMinEdges
+                           ? 0
+                           : light_edges(ctx, ctx->tune_light_per_vertex, plan.m, plan.n);
     a.light_k = k ? k : plan.m;
+    a.light_k2 = light_edges(ctx, 2 * ctx->tune_light_per_vertex, plan.m, plan.n);
+    if (!a.light_k2)
+        a.light_k2 = a.light_k;
     a.threshold = k && KIND == kKindPacked ? k : kKeyNone;
     a.nsamp = k && KIND == kKindMsf ? sample_count(plan.m) : 0;
-    const int threads = 256 * ctx->tune_edge_ctas;
-    const uint32_t blocks = solve_blocks(plan.m, ctx->sm_count);
-    a.seg = seg_records(plan.m, blocks * (uint32_t)(threads / 32), KIND == kKindMsf ? 12 : 8);
+    constexpr uint32_t rec_bytes = KIND == kKindMsf ? 12 : 8;
+    const SolveGrid g = solve_grid(plan.m, rec_bytes, ctx->sm_count, ctx->tune_edge_ctas);
+    a.seg = seg_records(plan.m, g.blocks * (uint32_t)(g.threads / 32), rec_bytes);
     PHEM_CUDA_TRY(cudaMemsetAsync(ctx->ctl, 0, sizeof(Ctl), st));
     void *params[] = {&a};
     KernelScope ks(ctx, kKSolve);
-    if (blocks == 1)  // one CTA waits for no other
-        PHEM_CUDA_TRY(cudaLaunchKernel(solve_kernel<KIND>, dim3(1), dim3(threads), params, sizeof(SolveSmem), st));
+    if (g.blocks == 1)  // one CTA waits for no other
+        PHEM_CUDA_TRY(cudaLaunchKernel(solve_kernel<KIND>, dim3(1), dim3(g.threads), params, sizeof(SolveSmem), st));
     else
-        PHEM_CUDA_TRY(cudaLaunchCooperativeKernel(solve_kernel<KIND>, dim3(blocks), dim3(threads), params,
+        PHEM_CUDA_TRY(cudaLaunchCooperativeKernel(solve_kernel<KIND>, dim3(g.blocks), dim3(g.threads), params,
                                                   sizeof(SolveSmem), st));
     return PHEM_OK;
 }
@@ -1234,7 +1280,7 @@ static size_t msf_carve(uint64_t m, uint32_t n, int sm_count, char *base, MsfPla
     Carve c;
     const uint64_t stride = ((uint64_t)n + 31) & ~31ull;
     const size_t o_par = c.take<uint32_t>(n), o_best = c.take<unsigned long long>(2 * stride),
-                 o_samp = c.take<uint32_t>(kMaxSample), o_bm = c.take<uint32_t>((m + 31) / 32 + 4),
+                 o_samp = c.take<uint32_t>(2 * kMaxSample), o_bm = c.take<uint32_t>((m + 31) / 32 + 4),
                  o_cnt = c.take<uint32_t>(gather_chunks(m) + 4), o_tot = c.take<uint32_t>(kMaxGrid),
                  o_gi = c.take<uint32_t>(stride / 32 + 4), o_list = c.take<uint4>(list_capacity(m, sm_count)),
                  o_hk = c.take<uint32_t>(list_capacity(m, sm_count));
