@@ -334,7 +334,9 @@ phem_status phem_csr_to_coo(phem_context *ctx, const int64_t *offsets, const uin
 /* ------------------------------------------------------------ batched small graphs */
 /* Many independent graphs solved in ONE persistent kernel launch: CTAs take
  * whole graphs from a device work queue (largest first) and run Boruvka on
- * each to completion.  No reference counterpart: the reference solves one
+ * each to completion; a batch whose largest graphs would keep one SM busy long
+ * after the others is solved as one disjoint union by the whole grid instead
+ * (the same results; the batch.* tuning then has no part).  No reference counterpart: the reference solves one
  * graph per call (boruvka_for_edge_array, MST/src/new_boruvka.cu:40-179),
  * and this is the batch of such calls without their launch overhead.  Every
  * graph gets exactly what the one-graph entry points give it:

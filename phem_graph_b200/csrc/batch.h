@@ -47,6 +47,33 @@ struct BatchArgs {
     float compact_ratio;         // compact a list pass when live <= ratio * length
 };
 
+// One graph as the grid kernel (batch_grid.cu) sees it.
+struct GridItem {
+    uint64_t e_off;   // first input record
+    uint32_t m, n;
+    uint32_t v_off;   // caller's vertex_offset: outputs
+    uint32_t kind, index;
+    uint32_t tile0;   // the graph's first tile of the union
+    uint32_t vb;      // the graph's first vertex of the union (a multiple of 32)
+    uint32_t skip;    // records between the first tile's aligned start and e_off
+};
+// Sizes of one launch of it (device memory, so one captured launch serves any
+// batch); items = 0: nothing to do.
+struct GridHdr {
+    uint32_t items, tiles, vertices, pad;
+};
+// Its device buffers.
+struct BatchGrid {
+    GridHdr *hdr = nullptr;  // one per launch: the whole batch's, then the groups'
+    GridItem *items = nullptr;
+    Ctl *ctl = nullptr;
+    void *tiles = nullptr;
+    uint32_t *vitem = nullptr, *parent = nullptr, *bitmap = nullptr, *tile_off = nullptr, *cta_tot = nullptr,
+             *hooked = nullptr;
+    unsigned long long *best = nullptr, *thr = nullptr;
+    uint64_t best_stride = 0;
+};
+
 struct BatchLaunch {
     const void *kernel = nullptr;
     int block = 0, items = 0, grid = 0;
@@ -100,6 +127,21 @@ size_t batch_carve(uint32_t G, uint64_t E, uint64_t wl, uint64_t bm, uint32_t V,
                    BatchBuffers *b);
 BatchArgs make_args(const BatchBuffers &b, const phem_edge *edges, float ratio);
 
+// ---- one union over the whole grid (batch_grid.cu) ----
+constexpr float kGridLightMsf = 1.f;  // light edges per vertex of a weighted graph
+// True when the batch goes to the grid kernel.
+bool batch_takes_grid(const BatchLayout &L, int sm_count);
+// List records its survivor segments need.
+uint64_t batch_grid_list(uint64_t records, uint32_t G, int sm_count);
+// Carves its buffers behind `off` (base null: sizing only); returns the end.
+size_t batch_grid_carve(uint32_t G, uint64_t records, uint32_t V, int sm_count, size_t off, char *base, BatchGrid *g);
+// The grid form of `items` (one launch's), and its sizes.
+GridHdr batch_grid_items(const BatchItem *items, uint32_t G, GridItem *out);
+// Queues launch `group` (its header) over the items from `first` on.
+phem_status batch_grid_launch(cudaStream_t stream, int sm_count, const BatchGrid &g, uint32_t group, uint32_t first,
+                              const phem_edge *edges, uint4 *list, const BatchArgs &b, float light_msf,
+                              float light_cc);
+
 // Resolves the kernel for (block, items), sets its shared-memory attribute and
 // sizes the persistent grid from the occupancy API.
 phem_status batch_launch_config(int device, int sm_count, int block, int items, BatchLaunch *out);
@@ -115,6 +157,9 @@ struct phem_batch_plan {
     phem::BatchBuffers buf{};
     phem::BatchLaunch launch{};
     float ratio = 0.5f;
+    phem::BatchGrid grid{};              // the grid kernel's buffers (null in a serving slot's plan)
+    phem::GridItem *h_grid = nullptr;    // pinned staging of its items
+    phem::GridHdr *h_hdr = nullptr;
     phem::BatchItem *h_items = nullptr;  // pinned staging of the work items
     uint32_t *h_num = nullptr;     // pinned batch size
     uint32_t *h_status = nullptr;  // pinned per-graph status
@@ -126,4 +171,9 @@ struct phem_batch_plan {
 
 namespace phem {
 phem_status batch_plan_capture(phem_batch_plan *p, const unsigned long long *pairs);
+// phem_batch_plan_create; with `grid` the plan can also route a batch to the
+// grid kernel (a serving slot's plan cannot: its launches overlap on the
+// device, and a cooperative launch waits for every SM).
+phem_status batch_plan_create(phem_context *ctx, uint32_t max_graphs, uint64_t max_edges, uint32_t max_vertices,
+                              bool grid, phem_batch_plan **out);
 }  // namespace phem

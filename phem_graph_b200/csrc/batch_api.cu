@@ -160,17 +160,22 @@ phem_status batch_status(const uint32_t *status, uint32_t G)
 // left for launch_overlapped to copy.
 phem_status batch_stage(phem_context *ctx, const phem_batch_graph *graphs, uint32_t G, const phem_edge *edges,
                         uint64_t E, uint32_t V, BatchLayout *L, BatchBuffers *b, const phem_edge **d_edges,
-                        BatchGroups *grp = nullptr)
+                        BatchGroups *grp = nullptr, BatchGrid *grid = nullptr)
 {
     PHEM_TRY(build_items(graphs, G, E, V, L));
+    const bool on_grid = grid && batch_takes_grid(*L, ctx->sm_count);
     if (E && !edges) {
         set_error("batch: null edge array");
         return PHEM_ERR_INVALID;
     }
     const bool dev_edges = E && is_device_ptr(edges) && ((uintptr_t)edges & 3) == 0;
-    const size_t bytes = batch_carve(G, E, L->wl_records, L->bm_words, V, !dev_edges, nullptr, nullptr);
-    PHEM_TRY(ws_reserve(ctx, bytes));
-    batch_carve(G, E, L->wl_records, L->bm_words, V, !dev_edges, static_cast<char *>(ctx->ws), b);
+    const uint64_t wl = on_grid ? batch_grid_list(L->wl_records, G, ctx->sm_count) : L->wl_records;
+    const size_t bytes = batch_carve(G, E, wl, L->bm_words, V, !dev_edges, nullptr, nullptr);
+    PHEM_TRY(ws_reserve(ctx, on_grid ? batch_grid_carve(G, L->wl_records, V, ctx->sm_count, bytes, nullptr, nullptr)
+                                     : bytes));
+    batch_carve(G, E, wl, L->bm_words, V, !dev_edges, static_cast<char *>(ctx->ws), b);
+    if (on_grid)
+        batch_grid_carve(G, L->wl_records, V, ctx->sm_count, bytes, static_cast<char *>(ctx->ws), grid);
     uint32_t nums[1 + kBatchGroups] = {G};
     if (grp && !dev_edges && E >= kBatchOverlapMinEdges && G >= 2) {
         grp->k = kBatchGroups;
@@ -195,10 +200,24 @@ phem_status batch_stage(phem_context *ctx, const phem_batch_graph *graphs, uint3
     } else if (grp) {
         grp->k = 0;
     }
-    if (G)
-        PHEM_CUDA_TRY(cudaMemcpyAsync(b->items, L->items.data(), sizeof(BatchItem) * G, cudaMemcpyHostToDevice,
+    if (on_grid) {
+        std::vector<GridItem> items(G);
+        GridHdr hdr[1 + kBatchGroups] = {};
+        if (grp && grp->k)
+            for (int k = 0; k < grp->k; k++)
+                hdr[1 + k] = batch_grid_items(L->items.data() + grp->start[k], grp->count[k],
+                                              items.data() + grp->start[k]);
+        else
+            hdr[0] = batch_grid_items(L->items.data(), G, items.data());
+        PHEM_CUDA_TRY(cudaMemcpyAsync(grid->items, items.data(), sizeof(GridItem) * G, cudaMemcpyHostToDevice,
                                       ctx->stream));
-    PHEM_CUDA_TRY(cudaMemcpyAsync(b->num_graphs, nums, sizeof(nums), cudaMemcpyHostToDevice, ctx->stream));
+        PHEM_CUDA_TRY(cudaMemcpyAsync(grid->hdr, hdr, sizeof(hdr), cudaMemcpyHostToDevice, ctx->stream));
+    } else {
+        if (G)
+            PHEM_CUDA_TRY(cudaMemcpyAsync(b->items, L->items.data(), sizeof(BatchItem) * G, cudaMemcpyHostToDevice,
+                                          ctx->stream));
+        PHEM_CUDA_TRY(cudaMemcpyAsync(b->num_graphs, nums, sizeof(nums), cudaMemcpyHostToDevice, ctx->stream));
+    }
     if (dev_edges) {
         *d_edges = edges;
     } else {
@@ -209,6 +228,14 @@ phem_status batch_stage(phem_context *ctx, const phem_batch_graph *graphs, uint3
     if (G)
         PHEM_CUDA_TRY(cudaMemsetAsync(b->rounds, 0, sizeof(uint32_t) * G, ctx->stream));
     return PHEM_OK;
+}
+
+// The whole batch, or group k of an overlapped one, on the grid kernel.
+phem_status launch_grid(phem_context *ctx, const BatchGrid &g, uint32_t hdr, uint32_t first, const BatchArgs &args)
+{
+    KernelScope k(ctx, kKBatch);
+    return batch_grid_launch(ctx->stream, ctx->sm_count, g, hdr, first, args.edges, args.wl, args, kGridLightMsf,
+                             (float)ctx->tune_canonical_light);
 }
 
 phem_status launch_once(phem_context *ctx, const BatchLaunch &l, const BatchArgs &args)
@@ -223,7 +250,7 @@ phem_status launch_once(phem_context *ctx, const BatchLaunch &l, const BatchArgs
 // only for it.
 phem_status launch_overlapped(phem_context *ctx, const BatchLaunch &l, const BatchArgs &args,
                               const BatchGroups &grp, const phem_edge *h_edges, phem_edge *d_edges,
-                              const BatchBuffers &b)
+                              const BatchBuffers &b, const BatchGrid &grid)
 {
     cudaEvent_t ev[kBatchGroups + 1] = {};
     phem_status st = PHEM_OK;
@@ -251,7 +278,9 @@ phem_status launch_overlapped(phem_context *ctx, const BatchLaunch &l, const Bat
             st = PHEM_ERR_CUDA;
             break;
         }
-        if (grp.count[k]) {
+        if (grp.count[k] && grid.hdr) {
+            st = launch_grid(ctx, grid, 1 + k, grp.start[k], args);
+        } else if (grp.count[k]) {
             BatchArgs a = args;
             a.items = args.items + grp.start[k];
             a.num_graphs = b.num_graphs + 1 + k;
@@ -301,21 +330,30 @@ phem_status batch_plan_capture(phem_batch_plan *p, const unsigned long long *pai
     *p->h_num = 0;
     cudaStream_t s = p->ctx->stream;
     cudaError_t e = cudaMemcpyAsync(p->buf.num_graphs, p->h_num, sizeof(uint32_t), cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess && p->grid.hdr)
+        e = cudaMemsetAsync(p->grid.hdr, 0, sizeof(GridHdr), s);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(s);
     if (e == cudaSuccess)
         e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
         const cudaError_t e1 = cudaMemsetAsync(p->buf.queue, 0, sizeof(uint32_t), s);
+        // a batch is either kernel's; the other one finds its size word zero
+        if (p->grid.hdr &&
+            batch_grid_launch(s, p->ctx->sm_count, p->grid, 0, 0, p->buf.edges, p->buf.wl,
+                              make_args(p->buf, p->buf.edges, p->ratio), kGridLightMsf,
+                              (float)p->ctx->tune_canonical_light) != PHEM_OK)
+            e = cudaErrorUnknown;
         BatchArgs a = make_args(p->buf, p->buf.edges, p->ratio);
         a.pairs = pairs;
         a.smem_vertices = p->launch.smem_vertices;
         void *params[] = {&a};
         const cudaError_t e2 = cudaLaunchKernel(p->launch.kernel, dim3(p->launch.grid), dim3(p->launch.block),
                                                 params, p->launch.dyn_smem, s);
+        const cudaError_t e0 = e;
         e = cudaStreamEndCapture(s, &p->graph);
         if (e == cudaSuccess)
-            e = e1 != cudaSuccess ? e1 : e2;
+            e = e0 != cudaSuccess ? e0 : (e1 != cudaSuccess ? e1 : e2);
     }
     if (e == cudaSuccess)
         e = cudaGraphInstantiate(&p->exec, p->graph, 0);
@@ -345,7 +383,8 @@ phem_status phem_batch_solve(phem_context *ctx, const phem_batch_graph *graphs, 
     BatchBuffers b{};
     const phem_edge *d_edges = nullptr;
     BatchGroups grp;
-    PHEM_TRY(batch_stage(ctx, graphs, num_graphs, edges, total_edges, total_vertices, &L, &b, &d_edges, &grp));
+    BatchGrid grid;
+    PHEM_TRY(batch_stage(ctx, graphs, num_graphs, edges, total_edges, total_vertices, &L, &b, &d_edges, &grp, &grid));
     BatchLaunch l;
     PHEM_TRY(batch_launch_config(ctx->device, ctx->sm_count, ctx->tune_batch_block, ctx->tune_batch_items, &l));
     const float ratio = (float)ctx->tune_batch_compact;
@@ -354,7 +393,9 @@ phem_status phem_batch_solve(phem_context *ctx, const phem_batch_graph *graphs, 
     {
         Timed timer(ctx);
         if (grp.k)
-            PHEM_TRY(launch_overlapped(ctx, l, args, grp, edges, b.edges, b));
+            PHEM_TRY(launch_overlapped(ctx, l, args, grp, edges, b.edges, b, grid));
+        else if (grid.hdr)
+            PHEM_TRY(launch_grid(ctx, grid, 0, 0, args));
         else
             PHEM_TRY(launch_once(ctx, l, args));
         ms = timer.stop();
@@ -453,6 +494,10 @@ void phem_batch_plan_destroy(phem_batch_plan *p)
         cudaEventDestroy(p->staged);
     if (p->h_items)
         cudaFreeHost(p->h_items);
+    if (p->h_grid)
+        cudaFreeHost(p->h_grid);
+    if (p->h_hdr)
+        cudaFreeHost(p->h_hdr);
     if (p->h_num)
         cudaFreeHost(p->h_num);
     if (p->h_status)
@@ -464,6 +509,14 @@ void phem_batch_plan_destroy(phem_batch_plan *p)
 
 phem_status phem_batch_plan_create(phem_context *ctx, uint32_t max_graphs, uint64_t max_edges, uint32_t max_vertices,
                                    phem_batch_plan **out)
+{
+    return batch_plan_create(ctx, max_graphs, max_edges, max_vertices, true, out);
+}
+
+}  // extern "C"
+
+phem_status phem::batch_plan_create(phem_context *ctx, uint32_t max_graphs, uint64_t max_edges, uint32_t max_vertices,
+                                    bool grid, phem_batch_plan **out)
 {
     PHEM_TRY(check_ctx(ctx));
     if (!out || max_graphs == 0) {
@@ -486,8 +539,10 @@ phem_status phem_batch_plan_create(phem_context *ctx, uint32_t max_graphs, uint6
     p->ratio = (float)ctx->tune_batch_compact;
     phem_status st = batch_launch_config(ctx->device, ctx->sm_count, ctx->tune_batch_block, ctx->tune_batch_items,
                                          &p->launch);
-    const size_t bytes = batch_carve(max_graphs, max_edges, p->max_wl, p->max_bm, max_vertices, true, nullptr,
-                                     nullptr);
+    const uint64_t wl = grid ? batch_grid_list(p->max_wl, max_graphs, ctx->sm_count) : p->max_wl;
+    const size_t core = batch_carve(max_graphs, max_edges, wl, p->max_bm, max_vertices, true, nullptr, nullptr);
+    const size_t bytes =
+        grid ? batch_grid_carve(max_graphs, p->max_wl, max_vertices, ctx->sm_count, core, nullptr, nullptr) : core;
     if (st == PHEM_OK && cudaMalloc(&p->mem, bytes) != cudaSuccess) {
         cudaGetLastError();
         p->mem = nullptr;
@@ -497,14 +552,18 @@ phem_status phem_batch_plan_create(phem_context *ctx, uint32_t max_graphs, uint6
     if (st == PHEM_OK && (cudaMallocHost(&p->h_items, sizeof(BatchItem) * max_graphs) != cudaSuccess ||
                           cudaMallocHost(&p->h_num, sizeof(uint32_t)) != cudaSuccess ||
                           cudaMallocHost(&p->h_status, sizeof(uint32_t) * max_graphs) != cudaSuccess ||
+                          (grid && (cudaMallocHost(&p->h_grid, sizeof(GridItem) * max_graphs) != cudaSuccess ||
+                                    cudaMallocHost(&p->h_hdr, sizeof(GridHdr)) != cudaSuccess)) ||
                           cudaEventCreateWithFlags(&p->staged, cudaEventDisableTiming) != cudaSuccess)) {
         cudaGetLastError();
         set_error("batch_plan_create: cannot allocate pinned staging");
         st = PHEM_ERR_NOMEM;
     }
     if (st == PHEM_OK) {
-        batch_carve(max_graphs, max_edges, p->max_wl, p->max_bm, max_vertices, true, static_cast<char *>(p->mem),
-                    &p->buf);
+        batch_carve(max_graphs, max_edges, wl, p->max_bm, max_vertices, true, static_cast<char *>(p->mem), &p->buf);
+        if (grid)
+            batch_grid_carve(max_graphs, p->max_wl, max_vertices, ctx->sm_count, core, static_cast<char *>(p->mem),
+                             &p->grid);
         st = phem::batch_plan_capture(p, nullptr);
     }
     if (st != PHEM_OK) {
@@ -514,6 +573,8 @@ phem_status phem_batch_plan_create(phem_context *ctx, uint32_t max_graphs, uint6
     *out = p;
     return PHEM_OK;
 }
+
+extern "C" {
 
 phem_status phem_batch_plan_upload(phem_batch_plan *p, const phem_batch_graph *graphs, uint32_t num_graphs,
                                    const phem_edge *edges, uint64_t total_edges, uint32_t total_vertices)
@@ -538,7 +599,17 @@ phem_status phem_batch_plan_upload(phem_batch_plan *p, const phem_batch_graph *g
     cudaStream_t s = p->ctx->stream;
     PHEM_CUDA_TRY(cudaEventSynchronize(p->staged));  // the previous upload's staging was consumed
     std::copy(L.items.begin(), L.items.end(), p->h_items);
-    *p->h_num = num_graphs;
+    // overlapping edge ranges can add up to more than the plan's edges: those
+    // batches stay with the CTA-per-graph kernel
+    const bool on_grid = p->grid.hdr && L.wl_records <= p->max_wl && batch_takes_grid(L, p->ctx->sm_count);
+    *p->h_num = on_grid ? 0 : num_graphs;
+    if (p->grid.hdr) {
+        *p->h_hdr = on_grid ? batch_grid_items(L.items.data(), num_graphs, p->h_grid) : GridHdr{};
+        PHEM_CUDA_TRY(cudaMemcpyAsync(p->grid.hdr, p->h_hdr, sizeof(GridHdr), cudaMemcpyHostToDevice, s));
+        if (on_grid)
+            PHEM_CUDA_TRY(cudaMemcpyAsync(p->grid.items, p->h_grid, sizeof(GridItem) * num_graphs,
+                                          cudaMemcpyHostToDevice, s));
+    }
     if (num_graphs)
         PHEM_CUDA_TRY(cudaMemcpyAsync(p->buf.items, p->h_items, sizeof(BatchItem) * num_graphs,
                                       cudaMemcpyHostToDevice, s));

@@ -253,7 +253,7 @@ struct MsfPlan {
     uint64_t best_stride;    // >= n
     uint32_t *samples;       // the threshold select's sampled weights
     uint32_t *bitmap;        // ceil(m / 32)
-    uint32_t *chunk_cnt;     // MSF edges per 1024 edge ids, then their offsets (gather)
+    uint32_t *chunk_off;     // offsets of the MSF edges of every 1024 edge ids (gather)
     uint32_t *cta_tot;       // forest edges per CTA's range (gather)
     uint32_t *giant;         // one bit per vertex
     uint4 *list;             // survivor segments, one per warp

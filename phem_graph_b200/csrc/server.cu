@@ -386,7 +386,8 @@ phem_status phem_server_create(int device, const phem_server_config *cfg, phem_s
         if (st == PHEM_OK)
             st = phem_context_create(device, &sl.ctx);
         if (st == PHEM_OK)
-            st = phem_batch_plan_create(sl.ctx, cfg->max_batch_graphs, s->slot_edges, s->slot_vertices, &sl.plan);
+            st = phem::batch_plan_create(sl.ctx, cfg->max_batch_graphs, s->slot_edges, s->slot_vertices, false,
+                                         &sl.plan);
         if (st == PHEM_OK && (cudaMalloc(&sl.d_pairs, 8 * s->slot_edges) != cudaSuccess ||
                               cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming) != cudaSuccess ||
                               cudaMallocHost(&sl.h_ids, 4 * (size_t)s->slot_vertices) != cudaSuccess ||

@@ -237,3 +237,63 @@ def test_full_workload_sampled(ctx):
         assert int(res.count[g]) == n - len(np.unique(res.graph_labels(b, g)))
     rng = np.random.default_rng(0)
     check_batch(b, res, graphs=sorted(rng.choice(b.num_graphs, 96, replace=False).tolist()))
+
+
+@pytest.mark.parametrize("device", [0, 1, 2])
+@pytest.mark.parametrize("kind", [gen.PHEM_BATCH_MSF, gen.PHEM_BATCH_CC])
+def test_grid_batch_shapes(ctx, device, kind):
+    """A batch with one graph large enough for the grid kernel, beside empty,
+    one-vertex, one-edge and tile-sized ones whose edges start at every offset
+    mod 4, with gaps and shared edge ranges, from host memory and from device
+    memory at 16- and 4-byte alignment."""
+    sizes = [(60000, 300001), (0, 0), (1, 0), (2, 1), (33, 127), (40, 128), (41, 129), (500, 1023), (7, 3), (3000, 9000)]
+    parts = []
+    for i, (n, m) in enumerate(sizes):
+        p = gen.er(n, m + m // 8 + 8, 50 + i)[:m] if m else np.zeros(0, np.uint64)
+        parts.append((f"g{i}", n, gen.msf_edges(p, gen.weights(len(p), i, bits=5)), kind))
+    b = gen.batch_from(parts)
+    # the second 127-edge graph reads the first one's records; vertex ranges get gaps
+    b.graphs[7]["edge_offset"] = b.graphs[4]["edge_offset"]
+    b.graphs[7]["num_edges"] = 127
+    b.graphs["vertex_offset"] += np.arange(len(sizes), dtype=np.uint32) * 5
+    b.total_vertices += 5 * len(sizes)
+    host = b.edges
+    if device:
+        import torch
+        t = torch.from_numpy(np.concatenate([host[:device - 1], host]).view(np.int32)).cuda()
+        torch.cuda.synchronize()
+        b.edges = t[device - 1:]
+    r = ctx.batch_solve(b)
+    for g in range(len(sizes)):
+        q = b.graphs[g]
+        o, m, n = int(q["edge_offset"]), int(q["num_edges"]), int(q["num_vertices"])
+        E = host[o:o + m].copy()
+        if kind == gen.PHEM_BATCH_CC:
+            E[:, 2] = 0
+        flags, cnt, tot = oracle.msf_kruskal(E, n) if n else (np.zeros(0), 0, 0)
+        assert (int(r.count[g]), int(r.total[g])) == (cnt, tot)
+        np.testing.assert_array_equal(r.forest(b, g), np.nonzero(flags)[0])
+        if n:
+            labels, _ = oracle.cc_solve((E[:, 0].astype(np.uint64) << np.uint64(32)) | E[:, 1], n)
+            np.testing.assert_array_equal(r.graph_labels(b, g), labels)
+
+
+def test_plan_replays_both_kernels(ctx):
+    """One plan, a batch for the CTA-per-graph kernel, one for the grid, and
+    the first again; a bad endpoint in the grid batch is reported."""
+    small, large = gen.mixed_batch(12, 5, 64, 300), gen.mixed_batch(6, 6, 20000, 40000)
+    with ctx.batch_plan(16, max(small.total_edges, large.total_edges), max(small.total_vertices, large.total_vertices)) as p:
+        for b in (small, large, small):
+            p.upload(b)
+            p.run()
+            r = p.download()
+            for g in range(b.num_graphs):
+                E, n = b.graph_edges(g), int(b.graphs[g]["num_vertices"])
+                flags, cnt, tot = oracle.msf_kruskal(E, n)
+                assert (int(r.count[g]), int(r.total[g])) == (cnt, tot)
+                np.testing.assert_array_equal(r.forest(b, g), np.nonzero(flags)[0])
+        large.edges[int(large.graphs[1]["edge_offset"]) + 3, 1] = 70000
+        p.upload(large)
+        p.run()
+        with pytest.raises(PhemError):
+            p.download()
