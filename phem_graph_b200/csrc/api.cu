@@ -9,7 +9,6 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
-#include <cstdlib>
 #include <thread>
 
 #include "internal.h"
@@ -23,7 +22,7 @@ thread_local char g_last_error[512] = "";
 }  // namespace
 
 const char *const kKernelNames[kKernelCount] = {
-    "msf_solve", "msf_init", "msf_select", "msf_edge_pass", "msf_hook", "msf_compress", "msf_gather",
+    "cc_solve", "msf_solve", "msf_init", "msf_select", "msf_edge_pass", "msf_hook", "msf_compress", "msf_gather",
     "cc_init", "cc_unite", "cc_merge", "cc_label", "cc_minid", "cc_count", "csr_to_coo", "batch_solve"};
 
 constexpr size_t kLaunchLogCap = 1u << 16;
@@ -650,7 +649,21 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
                  fb = (size_t)n * sizeof(uint64_t);
     // extra area: staged edges | labels | forest | parent (default path)
     const size_t o_edges = 0, o_lab = align256(eb), o_for = o_lab + align256(lb), o_par = o_for + align256(fb);
-    const size_t extra = o_par + align256(lb);
+    const bool on_device = is_device_ptr(edges);
+    const bool aligned_dev = on_device && (((uintptr_t)edges & 15) == 0);
+    // large host inputs of the default path are copied in chunks, overlapped
+    // with the unions of the chunks before them
+    const bool overlap = !canonical && !on_device && m >= kOverlapMinEdges;
+    // a prefix sample of about tune_cc_sample edges per vertex builds the big
+    // components, a compress points every vertex at its root, and the
+    // remaining edges then mostly settle with two loads
+    int64_t s = (int64_t)(ctx->tune_cc_sample * (double)n) & ~int64_t(3);
+    if (s <= 0 || s >= m)
+        s = m;
+    // edges on the device are solved in one launch, whose lists hold the
+    // prefix (a much longer one than usual stays with the launches below)
+    const bool one_launch = !canonical && !overlap && s <= 4 * (int64_t)n + (1 << 20);
+    const size_t extra = o_par + (one_launch ? cc_grid_bytes(m, s, n, ctx->sm_count) : align256(lb));
     size_t base = 0;
     MsfPlan plan;
     if (canonical) {
@@ -659,11 +672,6 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
         PHEM_TRY(ws_reserve(ctx, extra));
     }
     Staged se, sl, sf;
-    const bool on_device = is_device_ptr(edges);
-    const bool aligned_dev = on_device && (((uintptr_t)edges & 15) == 0);
-    // large host inputs of the default path are copied in chunks, overlapped
-    // with the unions of the chunks before them
-    const bool overlap = !canonical && !on_device && m >= kOverlapMinEdges;
     if (aligned_dev) {
         se.dev = const_cast<uint64_t *>(edges);
     } else {
@@ -685,16 +693,12 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
         PHEM_TRY(msf_run(ctx, kKindPacked, plan));
         // plan.best is free after the rounds: reuse it as the per-root min-id array
         PHEM_TRY(cc_launch_minid_labels(ctx, n, plan.parent, reinterpret_cast<uint32_t *>(plan.best), d_lab));
+    } else if (one_launch) {
+        PHEM_TRY(cc_grid(ctx, d_edges, m, s, n, d_lab, d_for, static_cast<char *>(ctx->ws) + base + o_par));
     } else {
         int32_t *d_par = reinterpret_cast<int32_t *>(static_cast<char *>(ctx->ws) + base + o_par);
         PHEM_CUDA_TRY(cudaMemsetAsync(ctx->ctl, 0, sizeof(Ctl), ctx->stream));
         PHEM_TRY(cc_launch_init(ctx, n, d_par, nullptr, d_for));
-        // a prefix sample of about tune_cc_sample edges per vertex builds the
-        // big components, a compress points every vertex at its root, and
-        // the remaining edges then mostly settle with two loads
-        int64_t s = (int64_t)(ctx->tune_cc_sample * (double)n) & ~int64_t(1);
-        if (s <= 0 || s >= m)
-            s = m;
         if (overlap) {
             PHEM_TRY(cc_unite_overlapped(ctx, edges, const_cast<uint64_t *>(d_edges), m, s, n, d_par, d_for));
         } else {
@@ -707,7 +711,8 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
         PHEM_TRY(cc_launch_label(ctx, n, d_par, d_lab));
     }
     cudaEventRecord(ctx->ev_stop, ctx->stream);
-    PHEM_TRY(cc_launch_count(ctx, n, d_lab, d_for));
+    if (!one_launch)
+        PHEM_TRY(cc_launch_count(ctx, n, d_lab, d_for));
     PHEM_TRY(copy_back(ctx, sl, lb));
     PHEM_TRY(copy_back(ctx, sf, fb));
     PHEM_TRY(msf_finish(ctx, &rounds, "cc_solve"));
@@ -716,7 +721,8 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
         ms = 0.f;
     if (stats) {
         stats->components = (uint32_t)ctx->h_ctl->misc[0];
-        stats->forest_edges = d_for ? ctx->h_ctl->misc[1] : (uint64_t)n - ctx->h_ctl->misc[0];
+        stats->forest_edges =
+            d_for && !one_launch ? ctx->h_ctl->misc[1] : (uint64_t)n - ctx->h_ctl->misc[0];
         stats->rounds = rounds;
         stats->device_ms = ms;
     }
@@ -1005,7 +1011,6 @@ static phem_status msf_tiny(phem_context *ctx, const phem_edge *edges, uint64_t 
     PHEM_TRY(tiny_msf(ctx, static_cast<const phem_edge *>(in), (uint32_t)m, n, out, d_count_total));
     cudaEventRecord(ctx->ev_stop, ctx->stream);
     PHEM_TRY(stream_wait(ctx));
-    if(getenv("PHEM_ST")) {for(uint32_t q=0;q<ctx->h_ctl->stamps;q++) printf("%.2f ",(double)ctx->h_ctl->stamp[q]/1900.); printf("\n");fflush(stdout);}
     PHEM_TRY(ctl_status(ctx->h_ctl->err, "msf"));
     if (host)
         std::memcpy(msf, out, ctx->h_ctl->msf_count * sizeof(phem_edge));

@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) batch_grid_kernel(const __gr
         }
         acc_add(s, lane == 0 ? filtered : 0u);
     }
-    if (!grid_sync(a.s, s, seq))
+    if (!grid_sync(ctl, s, seq))
         return give_up();
     const bool filter = s.sum > 0;
     uint32_t r = 0, src = kSrcLight;
@@ -345,23 +345,23 @@ __global__ void __launch_bounds__(kSolveThreads, 1) batch_grid_kernel(const __gr
         else
             grid_input_pass<false>(a, s, best, T, ws);
         offers_flush(s.oc, best);
-        if (!grid_sync(a.s, s, seq))
+        if (!grid_sync(ctl, s, seq))
             return give_up();
         r++;
         if (s.sum > 0) {
             hook_pass<kKindMsf>(a.s, s, best, next, ws);
-            if (!grid_sync(a.s, s, seq))
+            if (!grid_sync(ctl, s, seq))
                 return give_up();
-            compress_pass(a.s, ws);
+            compress_pass(a.s.parent, a.s.n, &ctl->err, ws);
             src = kSrcList;
         } else {
             if (heavy || !filter)
                 break;
-            full_compress(a.s, V, next, 0, false);
+            full_compress(a.s.parent, V, next, nullptr, 0, false, &ctl->err);
             heavy = true;
             src = kSrcHeavy;
         }
-        if (!grid_sync(a.s, s, seq))
+        if (!grid_sync(ctl, s, seq))
             return give_up();
         if (r >= PHEM_MAX_ROUNDS) {
             if (blockIdx.x == 0 && tid == 0)
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) batch_grid_kernel(const __gr
     // every vertex to its root; the roots' words of `mins` start the minimum
     // vertex ids; the tiles' forest counts become offsets
     unsigned long long *mins = a.s.best;
-    full_compress(a.s, V, mins, 0, false);
+    full_compress(a.s.parent, V, mins, nullptr, 0, false, &ctl->err);
     const uint64_t per = max((T + gridDim.x - 1) / gridDim.x, 1u);
     count_scan(s, a.s.chunk_off, T, per, a.s.cta_tot, [&](uint64_t, uint64_t i, uint64_t end) {
         if (i >= end)
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) batch_grid_kernel(const __gr
         const uint4 b = __ldcg(reinterpret_cast<const uint4 *>(a.s.bitmap) + i);
         return (uint32_t)(__popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w));
     });
-    if (!grid_sync(a.s, s, seq))
+    if (!grid_sync(ctl, s, seq))
         return give_up();
     const uint32_t all = prefix_totals(s, a.s.cta_tot);
     if (tid == 0)
@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) batch_grid_kernel(const __gr
         if ((int)lane == __ffs(peers) - 1 && x < __ldcg(minid + 2 * (uint64_t)root))
             atomicMin(minid + 2 * (uint64_t)root, x);
     }
-    if (!grid_sync(a.s, s, seq))
+    if (!grid_sync(ctl, s, seq))
         return give_up();
     for (uint32_t q = ws.gw; q < V / 32; q += ws.GW) {
         const GridItem &it = a.items[__ldcg(a.vitem + q)];

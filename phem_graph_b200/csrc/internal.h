@@ -14,7 +14,8 @@
 namespace phem {
 // Kernels the library launches; the profile reports them by these names.
 enum KernelId : int {
-    kKSolve = 0,  // the MSF solve; the next six are its phases (device timestamps, no launches)
+    kKCcSolve = 0,  // the one-launch CC solve; phases: kKCcInit, kKCcUnite, kKCcLabel
+    kKSolve,        // the MSF solve; the next six are its phases (device timestamps, no launches)
     kKInit, kKSelect, kKEdgePass, kKHook, kKCompress, kKGather,
     kKCcInit, kKCcUnite, kKCcMerge, kKCcLabel, kKMinid, kKCcCount, kKCsrCoo, kKBatch,
     kKernelCount
@@ -287,6 +288,20 @@ phem_status cc_launch_merge(phem_context *ctx, const uint64_t *fa, const uint64_
 phem_status cc_launch_minid_labels(phem_context *ctx, int32_t n, uint32_t *parent, uint32_t *minid,
                                    int32_t *label);
 phem_status cc_launch_count(phem_context *ctx, int32_t n, const int32_t *label, const uint64_t *forest);
+
+// ---- CC in one launch (cc_grid.cu) ----
+struct SolveGrid {
+    uint32_t blocks;
+    int threads;
+};
+constexpr uint32_t kCcGridReady = 1u << 8;  // bit of phem_context::kernels_ready
+SolveGrid cc_grid_size(int64_t m, int sm_count);
+size_t cc_grid_bytes(int64_t m, int64_t s, int32_t n, int sm_count);
+// Queues the whole solve over device edges (16-byte aligned; s a multiple of
+// four unless s = m): labels, forest slots (may be null), and the number of
+// components in ctx->ctl->misc[0].
+phem_status cc_grid(phem_context *ctx, const uint64_t *d_edges, int64_t m, int64_t s, int32_t n, int32_t *d_labels,
+                    uint64_t *d_forest, void *ws);
 
 // ---- CSR (csr.cu) ----
 // Device scratch the conversion needs for nnz entries (per-tile rows, counts

@@ -444,18 +444,8 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(const __grid_co
     Ctl *ctl = a.ctl;
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5, nw = blockDim.x >> 5;
     const bool lead = blockIdx.x == 0 && tid == 0;
-    uint32_t seq = 0, marks = 0;
-    auto stamp = [&](uint32_t phase) {
-        if (a.timing && lead && marks < kMaxPhases) {
-            uint64_t t;
-            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-            ctl->stamp[marks] = t;
-            ctl->phase_of[marks] = phase;
-            marks++;
-            ctl->stamps = marks;
-        }
-    };
-    stamp(kKernelCount);
+    uint32_t seq = 0;
+    PhaseClock clock(ctl, a.timing);
     // init
     {
         const uint64_t g = (uint64_t)blockIdx.x * blockDim.x + tid, T = (uint64_t)gridDim.x * blockDim.x;
@@ -481,13 +471,13 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(const __grid_co
         }
         offers_reset(s.oc);
     }
-    if (!grid_sync(a, s, seq))
+    if (!grid_sync(ctl, s, seq))
         return;
-    stamp(kKInit);
+    clock.stamp(kKInit);
     unsigned long long thr = a.threshold;
     if (a.nsamp) {
         thr = select_threshold(a, s);
-        stamp(kKSelect);
+        clock.stamp(kKSelect);
     }
     if (lane == 0) {  // after the select, whose samples shared this space
         for (int q = 0; q < kEpStages; q++)
@@ -514,23 +504,23 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(const __grid_co
         else
             input_pass<KIND, false>(a, s, best, thr, use_giant, ws);
         offers_flush(s.oc, best);
-        if (!grid_sync(a, s, seq))
+        if (!grid_sync(ctl, s, seq))
             return;
         const unsigned long long live = s.sum;
-        stamp(kKEdgePass);
+        clock.stamp(kKEdgePass);
         if (lead)
             ctl->m_r[r] = live;
         if (live > 0) {
             hook_pass<KIND>(a, s, best, next, ws);
-            if (!grid_sync(a, s, seq))
+            if (!grid_sync(ctl, s, seq))
                 return;
             if (lead)
                 ctl->n_r[r] = s.sum;
-            stamp(kKHook);
-            compress_pass(a, ws);
-            if (!grid_sync(a, s, seq))
+            clock.stamp(kKHook);
+            compress_pass(a.parent, a.n, &ctl->err, ws);
+            if (!grid_sync(ctl, s, seq))
                 return;
-            stamp(kKCompress);
+            clock.stamp(kKCompress);
             src = kSrcList;
         } else {
             if (light_rounds) {  // the heavy phase ran dry
@@ -544,10 +534,10 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(const __grid_co
             }
             uint32_t giant = 0;
             use_giant = a.n >= kGiantMinN && find_giant(a, s, KIND == kKindPacked, &giant);
-            full_compress(a, a.n, next, giant, use_giant);
-            if (!grid_sync(a, s, seq))
+            full_compress(a.parent, a.n, next, a.giant, giant, use_giant, &ctl->err);
+            if (!grid_sync(ctl, s, seq))
                 return;
-            stamp(kKCompress);
+            clock.stamp(kKCompress);
             src = kSrcHeavy;
         }
         if (++r >= PHEM_MAX_ROUNDS) {
@@ -578,10 +568,10 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(const __grid_co
             }
             return mine;
         });
-        if (!grid_sync(a, s, seq))
+        if (!grid_sync(ctl, s, seq))
             return;
         gather_pass(a, s, per);
-        stamp(kKGather);
+        clock.stamp(kKGather);
     }
 }
 
@@ -629,10 +619,6 @@ phem_status setup_kernel(phem_context *ctx)
 // among fewer warps), a large one needs the warps.  us per solve with 256 /
 // 512 / 1024 threads: m = 100,003 137 / 138 / 161; m = 200,000 183 / 163 /
 // 198; m = 2^20 250 / 238 / 250; m = 4,000,000 442 / 373 / 361.
-struct SolveGrid {
-    uint32_t blocks;
-    int threads;
-};
 SolveGrid solve_grid(uint64_t m, uint32_t rec_bytes, int sm_count, int max_groups)
 {
     const uint64_t tile = kEpStageBytes / rec_bytes, tiles = (m + tile - 1) / tile;

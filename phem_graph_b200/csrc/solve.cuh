@@ -115,7 +115,8 @@ static_assert(sizeof(EpWarp) * kSolveWarps >= (kMaxSample + kSeenWords) * sizeof
 // barrier see every store made before it on any SM.  1.2 us on 148 CTAs.
 constexpr uint32_t kBarSpinCap = 1u << 22;  // about 3 s
 
-__device__ __forceinline__ bool grid_sync(const SolveArgs &a, SolveSmem &s, uint32_t &seq)
+template <class Smem>
+__device__ __forceinline__ bool grid_sync(Ctl *ctl, Smem &s, uint32_t &seq)
 {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -123,12 +124,12 @@ __device__ __forceinline__ bool grid_sync(const SolveArgs &a, SolveSmem &s, uint
         s.acc = 0;
         __threadfence();
         if (gridDim.x > 1) {
-            unsigned long long *word = &a.ctl->bar[seq];
+            unsigned long long *word = &ctl->bar[seq];
             v += atomicAdd(word, v + (1ull << 52)) + (1ull << 52);
             uint32_t spins = 0;
             while ((v >> 52) < gridDim.x) {
                 if (++spins > kBarSpinCap) {
-                    set_err(&a.ctl->err, kErrLookback);
+                    set_err(&ctl->err, kErrLookback);
                     v |= 1ull << 40;
                     break;
                 }
@@ -143,6 +144,27 @@ __device__ __forceinline__ bool grid_sync(const SolveArgs &a, SolveSmem &s, uint
     seq++;
     return s.abort == 0;
 }
+
+// Profiling: one thread of the grid stamps the end of each phase.
+struct PhaseClock {
+    Ctl *ctl;
+    uint32_t marks = 0;
+    bool on;
+    __device__ PhaseClock(Ctl *c, int timing) : ctl(c), on(timing && blockIdx.x == 0 && threadIdx.x == 0)
+    {
+        stamp(kKernelCount);  // the start
+    }
+    __device__ __forceinline__ void stamp(uint32_t phase)
+    {
+        if (!on || marks >= kMaxPhases)
+            return;
+        uint64_t t;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+        ctl->stamp[marks] = t;
+        ctl->phase_of[marks] = phase;
+        ctl->stamps = ++marks;
+    }
+};
 
 // parent[] through L1 (weak, never the read-only path: this kernel writes it).
 __device__ __forceinline__ uint32_t ld_par(const uint32_t *p)
@@ -159,7 +181,8 @@ __device__ __forceinline__ unsigned long long ld_best(const unsigned long long *
 }
 
 // Adds a per-lane count to the CTA's contribution to the next barrier.
-__device__ __forceinline__ void acc_add(SolveSmem &s, uint32_t v)
+template <class Smem>
+__device__ __forceinline__ void acc_add(Smem &s, uint32_t v)
 {
     v = __reduce_add_sync(0xffffffffu, v);
     if (lane_id() == 0 && v)
@@ -392,7 +415,7 @@ __device__ __forceinline__ void hook_pass(const SolveArgs &a, SolveSmem &s, cons
 // L2, where the other lanes' shortcuts are.
 constexpr int kVItems = 4;
 
-__device__ __forceinline__ void compress_pass(const SolveArgs &a, const WarpState &ws)
+__device__ __forceinline__ void compress_pass(uint32_t *parent, uint32_t n, uint32_t *err, const WarpState &ws)
 {
     for (uint32_t i0 = lane_id(); i0 < ws.hooks; i0 += 32 * kVItems) {
         uint32_t x[kVItems], y[kVItems];
@@ -404,25 +427,25 @@ __device__ __forceinline__ void compress_pass(const SolveArgs &a, const WarpStat
         }
 #pragma unroll
         for (int k = 0; k < kVItems; k++)
-            y[k] = walking[k] ? ld_par(a.parent + x[k]) : 0u;
+            y[k] = walking[k] ? ld_par(parent + x[k]) : 0u;
         for (uint32_t steps = 0;; steps++) {
             uint32_t p[kVItems];
 #pragma unroll
             for (int k = 0; k < kVItems; k++)
-                p[k] = !walking[k] ? y[k] : (steps < 8 ? ld_par(a.parent + y[k]) : __ldcg(a.parent + y[k]));
+                p[k] = !walking[k] ? y[k] : (steps < 8 ? ld_par(parent + y[k]) : __ldcg(parent + y[k]));
             bool any = false;
 #pragma unroll
             for (int k = 0; k < kVItems; k++) {
                 walking[k] = walking[k] && p[k] != y[k];
                 if (walking[k])
-                    a.parent[x[k]] = p[k];
+                    parent[x[k]] = p[k];
                 y[k] = p[k];
                 any |= walking[k];
             }
             if (!any)
                 break;
-            if (steps > a.n) {
-                set_err(&a.ctl->err, kErrChase);
+            if (steps > n) {
+                set_err(err, kErrChase);
                 break;
             }
         }
@@ -430,10 +453,13 @@ __device__ __forceinline__ void compress_pass(const SolveArgs &a, const WarpStat
 }
 
 // Vertices [0, n) pointed at their roots (before the heavy pass, which then
-// relabels endpoints in one hop) and the roots' next best words reset; with
-// use_giant also one bit per vertex: in the component of root `giant`.
-__device__ __forceinline__ void full_compress(const SolveArgs &a, uint32_t n, unsigned long long *best_next,
-                                              uint32_t giant, bool use_giant)
+// relabels endpoints in one hop) and the roots' next best words reset (when
+// best_next is set); with use_giant also one bit per vertex: in the component
+// of root `giant`; with forest also every vertex's forest slot, the edge to
+// the parent it had.
+__device__ __forceinline__ void full_compress(uint32_t *parent, uint32_t n, unsigned long long *best_next,
+                                              uint32_t *bits_of, uint32_t giant, bool use_giant, uint32_t *err,
+                                              unsigned long long *forest = nullptr)
 {
     const uint32_t lane = lane_id();
     const uint64_t step = (uint64_t)gridDim.x * blockDim.x * kVItems;
@@ -450,12 +476,12 @@ __device__ __forceinline__ void full_compress(const SolveArgs &a, uint32_t n, un
         }
 #pragma unroll
         for (int k = 0; k < kVItems; k++)
-            y0[k] = y[k] = ld_par(a.parent + x[k]);
+            y0[k] = y[k] = ld_par(parent + x[k]);
         for (uint32_t steps = 0;; steps++) {
             uint32_t p[kVItems];
 #pragma unroll
             for (int k = 0; k < kVItems; k++)
-                p[k] = walking[k] ? ld_par(a.parent + y[k]) : y[k];
+                p[k] = walking[k] ? ld_par(parent + y[k]) : y[k];
             bool any = false;
 #pragma unroll
             for (int k = 0; k < kVItems; k++) {
@@ -465,8 +491,8 @@ __device__ __forceinline__ void full_compress(const SolveArgs &a, uint32_t n, un
             }
             if (!any)
                 break;
-            if (steps > a.n) {
-                set_err(&a.ctl->err, kErrChase);
+            if (steps > n) {
+                set_err(err, kErrChase);
                 break;
             }
         }
@@ -474,15 +500,17 @@ __device__ __forceinline__ void full_compress(const SolveArgs &a, uint32_t n, un
         for (int k = 0; k < kVItems; k++) {
             const uint64_t i = i0 + k * blockDim.x + threadIdx.x;
             if (i < n) {
+                if (forest)
+                    forest[i] = y0[k] != x[k] ? (unsigned long long)y0[k] << 32 | i : kForestEmpty;
                 if (y0[k] != y[k])
-                    a.parent[x[k]] = y[k];
-                if (y[k] == x[k])
+                    parent[x[k]] = y[k];
+                if (best_next && y[k] == x[k])
                     best_next[x[k]] = kKeyNone;
             }
             if (use_giant) {  // blockDim.x and i0 are multiples of 32
                 const unsigned bits = __ballot_sync(0xffffffffu, i < n && y[k] == giant);
                 if (lane == 0 && i < n)
-                    a.giant[i >> 5] = bits;
+                    bits_of[i >> 5] = bits;
             }
         }
     }

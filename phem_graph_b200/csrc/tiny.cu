@@ -532,7 +532,7 @@ phem_status tiny_cc(phem_context *ctx, const uint64_t *d_edges, uint32_t m, uint
     a.labels = d_labels;
     a.forest = reinterpret_cast<unsigned long long *>(d_forest);
     a.res = ctx->h_ctl;
-    KernelScope ks(ctx, kKCcUnite);
+    KernelScope ks(ctx, kKCcSolve);
     return launch(ctx, tiny_cc_kernel, 6, a, (size_t)n * 4 + 16);
 }
 

@@ -106,18 +106,10 @@ __device__ __forceinline__ bool uf_find2(int32_t *parent, int32_t a, int32_t b, 
 
 // One union with the reference's hook rule (larger root under smaller root,
 // forest[hooked root] = edge).  Returns true when it hooked.
-__device__ __forceinline__ bool uf_unite(int32_t *parent, unsigned long long *forest, unsigned long long e,
-                                         int32_t u, int32_t v, int32_t n, uint32_t *err)
+// u and v: the endpoints, or ancestors of theirs.
+__device__ __forceinline__ bool uf_unite_from(int32_t *parent, unsigned long long *forest, unsigned long long e,
+                                              int32_t u, int32_t v, int32_t n, uint32_t *err)
 {
-    {
-        // two independent loads settle most edges once parents point at roots
-        // (after a compress): equal parents mean one component
-        const int32_t pu = ld_ca(parent + u), pv = ld_ca(parent + v);
-        if (pu == pv)
-            return false;
-        u = pu;  // ancestors of the endpoints
-        v = pv;
-    }
     for (uint32_t retry = 0; retry < kUnionRetryCap; retry++) {
         // first attempt through L1; after a failed CAS, coherent walks
         int32_t ru, rv;
@@ -141,6 +133,15 @@ __device__ __forceinline__ bool uf_unite(int32_t *parent, unsigned long long *fo
     }
     set_err(err, kErrRetry);
     return false;
+}
+
+__device__ __forceinline__ bool uf_unite(int32_t *parent, unsigned long long *forest, unsigned long long e,
+                                         int32_t u, int32_t v, int32_t n, uint32_t *err)
+{
+    // two independent loads settle most edges once parents point at roots
+    // (after a compress): equal parents mean one component
+    const int32_t pu = ld_ca(parent + u), pv = ld_ca(parent + v);
+    return pu != pv && uf_unite_from(parent, forest, e, pu, pv, n, err);
 }
 
 __device__ __forceinline__ void unite_packed(int32_t *parent, unsigned long long *forest, unsigned long long e,

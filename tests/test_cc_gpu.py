@@ -322,3 +322,41 @@ def test_solves_from_reference_file_formats(ctx, tmp_path):
     r = ctx.msf_solve(e, n)
     assert (r.count, r.total) == (cnt, tot)
     np.testing.assert_array_equal(r.edges, e[flags])
+
+
+@pytest.mark.parametrize("kind", ["er", "er_long_rest", "rmat", "rgg", "path", "path_shuffled", "star_low", "star_high"])
+@pytest.mark.parametrize("odd", [0, 1])
+def test_device_edges_in_rounds(ctx, kind, odd):
+    """Device-resident edges past the one-CTA sizes: prefixes with and without
+    a rest, long chains, hubs as the smaller and as the larger endpoint of
+    repeated edges, odd counts; labels exact, slots exactly the non-roots, the
+    forest valid; out-of-range endpoints in the prefix and in the rest."""
+    import torch
+    n = 50001
+    u = np.arange(n - 1, dtype=np.uint64)
+    p = {"er": lambda: gen.er(n, 120000, 3), "er_long_rest": lambda: gen.er(n, 12 * n, 4),
+         "rmat": lambda: gen.rmat_graph(15, 16, seed=5).pairs, "rgg": lambda: gen.rgg_graph(n, 8, 3).pairs,
+         "path": lambda: (u << np.uint64(32)) | (u + np.uint64(1)),
+         "path_shuffled": lambda: np.random.default_rng(0).permutation((u << np.uint64(32)) | (u + np.uint64(1))),
+         "star_low": lambda: np.concatenate([u + np.uint64(1)] * 8),
+         "star_high": lambda: np.concatenate([(u << np.uint64(32)) | np.uint64(n - 1)] * 8)}[kind]()
+    p = np.ascontiguousarray(p[:len(p) - odd])
+    d = torch.from_numpy(p.view(np.int64)).cuda()
+    lab = torch.empty(n, dtype=torch.int32, device="cuda")
+    slots = torch.empty(n, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    r = ctx.cc_solve(d, n, labels=lab, forest=slots)
+    want, _ = oracle.cc_solve(p, n)
+    np.testing.assert_array_equal(lab.cpu().numpy(), want)
+    f = slots.cpu().numpy().view(np.uint64)
+    assert r.components == len(np.unique(want)) == n - r.forest_edges
+    np.testing.assert_array_equal(np.nonzero(f != np.uint64(_lib.PHEM_FOREST_EMPTY))[0],
+                                  np.nonzero(want != np.arange(n))[0])
+    check_forest(p, n, want, f)
+    for at in (5, len(p) - 1):
+        bad = d.clone()
+        bad[at] = (3 << 32) | n
+        torch.cuda.synchronize()
+        with pytest.raises(P.PhemError) as ei:
+            ctx.cc_solve(bad, n, labels=lab, forest=slots)
+        assert ei.value.status == _lib.PHEM_ERR_INVALID
