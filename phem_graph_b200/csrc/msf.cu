@@ -270,8 +270,12 @@ __device__ __forceinline__ void input_pass(const SolveArgs &a, SolveSmem &s, uns
     constexpr uint32_t TILE = kEpStageBytes / REC;
     const uint32_t lane = lane_id();
     EpWarp &w = s.warp[threadIdx.x >> 5];
-    const uint64_t ntiles = (a.m + TILE - 1) / TILE;
-    const uint64_t full_tiles = a.m / TILE;  // the partial last tile is read directly
+    // packed pairs are light by position: each pass reads its side of the list
+    const bool split = KIND == kKindPacked && thr != kKeyNone;
+    const uint64_t begin = !LIGHT && split ? thr / TILE : 0;
+    const uint64_t ntiles = LIGHT && split ? (thr + TILE - 1) / TILE : (a.m + TILE - 1) / TILE;
+    const uint64_t full_tiles = min(a.m / TILE, ntiles);  // the partial last tile is read directly
+    const uint64_t first = begin + ws.gw;
     const uint64_t policy = l2_evict_first();
     const char *src = static_cast<const char *>(a.e0);
     auto issue = [&](uint64_t t, int st) {  // lane 0 only
@@ -279,13 +283,13 @@ __device__ __forceinline__ void input_pass(const SolveArgs &a, SolveSmem &s, uns
         bulk_copy_g2s_hint(w.stage[st], src + t * kEpStageBytes, kEpStageBytes,
                            reinterpret_cast<uint64_t *>(&w.bar[st]), policy);
     };
-    if (lane == 0 && ws.gw < full_tiles)
-        issue(ws.gw, 0);
+    if (lane == 0 && first < full_tiles)
+        issue(first, 0);
     uint32_t filled = 0, flushed = 0;  // ring cursors (warp-uniform)
-    uint32_t pending = ws.gw < full_tiles ? 1u : 0u;  // bit s: a copy into stage s is in flight
+    uint32_t pending = first < full_tiles ? 1u : 0u;  // bit s: a copy into stage s is in flight
     bool any_bad = false, failed = false;
     int st = 0;
-    for (uint64_t t = ws.gw; t < ntiles; t += ws.GW, st ^= 1) {
+    for (uint64_t t = first; t < ntiles; t += ws.GW, st ^= 1) {
         // tile t + GW goes into the other stage, which the previous tile left
         // (its reads were fenced against the async proxy before the warp
         // synchronised at the end of that tile)
@@ -321,7 +325,7 @@ __device__ __forceinline__ void input_pass(const SolveArgs &a, SolveSmem &s, uns
     } else if (filled != flushed) {
         ring_flush<KIND>(a, s, best, ws.list, w, flushed, filled - flushed, lane);
     }
-    if (LIGHT && __any_sync(0xffffffffu, any_bad) && lane == 0)
+    if ((LIGHT || split) && __any_sync(0xffffffffu, any_bad) && lane == 0)
         set_err(&a.ctl->err, kErrRange);
     ws.len = flushed;
     acc_add(s, lane == 0 ? flushed : 0u);
