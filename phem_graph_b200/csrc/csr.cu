@@ -1,30 +1,33 @@
 // csr.cu -- symmetrised CSR -> packed COO (or {u, v, w} records) on sm_100a.
 //
 // csr_to_coo (CC/graph.cu:149-196) walks rows in order and emits (i << 32 | col)
-// for every entry with i < col.  Here the entries are cut into tiles of
-// kCsrTile consecutive entries on a static grid-stride schedule (no block
-// waits for another, so the loads of independent tiles overlap freely); a
-// tile is kCsrWarps segments of 256 entries, one per warp, read lane-striped
-// (step k of lane L holds entry 32k + L of the segment, so every load and
-// store is one contiguous warp access):
-//   1. csr_tile_rows_kernel, one thread per row, writes for every tile the row
-//      that holds its first entry, so no tile searches the offsets;
-//   2. csr_count_kernel marks, in shared memory, where each row inside the
-//      tile starts (one coalesced pass over the tile's offsets) together with
-//      the row each warp segment starts in; a warp then resolves the row of
-//      every entry with one ballot per step (the latest mark at or before the
-//      lane) and counts the entries with row < col;
-//   3. csr_scan_kernel turns the tile counts into tile offsets: every block
-//      scans a group of 4096 tiles and the last block to finish scans the
-//      groups' totals (no block waits for another);
-//   4. csr_write_kernel resolves the rows again and writes the kept entries in
-//      order: group offset + tile offset + the warps before + the lanes before
-//      (ballot).
+// for every entry with i < col.  Here the entries are cut into segments of 256
+// consecutive entries, each handled by one warp on its own -- no block
+// barrier anywhere -- with eight consecutive entries per lane:
+//   1. csr_seg_rows_kernel writes for every segment the row that holds its
+//      first entry, so no segment searches the offsets;
+//   2. csr_pass_kernel<kCount>: a warp marks, in its shared memory, where each
+//      row inside its segment starts, resolves the row of every entry from the
+//      marks and counts the entries with row < col;
+//   3. csr_scan_kernel turns the counts into offsets: every block scans a group
+//      of 4096 segments and the last block to finish scans the groups' totals
+//      (no block waits for another);
+//   4. csr_pass_kernel<kPairs or kRecords> resolves the rows again and writes
+//      the kept entries in order: group offset + segment offset + the lanes
+//      before.  The record form fuses the MSF CSR input's packing: the
+//      kept entry at position p becomes {row, col, w[p]}; a warp's records are
+//      put together in shared memory and leave as 16-byte stores.
 // Every entry keeps its place in the reference's row walk, so the output order
-// (and therefore the edge numbering) is exactly the reference's.  The record
-// form fuses the MSF CSR input's packing: the kept entry at position p becomes
-// {row, col, w[p]}.  Passes 2 and 4 load the next tile's columns and row
-// range while they work on the current one.
+// (and therefore the edge numbering) is exactly the reference's.  The next
+// segment's columns and row range are loaded while the current one is worked
+// on.
+//
+// R-MAT 20 (33.5 M entries; 134 MB read by pass 2, 402 MB moved by pass 4), us
+// of passes 1-4: 18 / 50 / 10 / 103 (13 / 72 / 9 / 148 with a block per 2048
+// entries, two block barriers each and 4-byte stores).  Bound: the latency of
+// the offsets' loads (without the marks pass 2 takes 31), above all in the
+// segments at the end that span up to 2,000 nearly empty rows.  A decoupled
+// look-back over 740 running blocks instead of passes 2 and 3: 2480.
 #include <algorithm>
 
 #include "internal.h"
@@ -32,158 +35,247 @@
 namespace phem {
 namespace {
 
-constexpr int kCsrThreads = 256;                  // threads per block of passes 2 and 4
+constexpr int kCsrThreads = 256;
 constexpr int kCsrWarps = kCsrThreads / 32;
-constexpr int kCsrItems = 8;                      // entries per lane per tile
-constexpr int kCsrSeg = 32 * kCsrItems;           // 256 entries per warp segment
-constexpr int kCsrTile = kCsrWarps * kCsrSeg;     // 2048 entries per tile
-constexpr int kCsrBlocksPerSm = 6;                // resident blocks per SM: 48 warps (registers <= 42)
+constexpr int kCsrItems = 8;           // entries per lane
+constexpr int kCsrSeg = 32 * kCsrItems;
+// Blocks per SM: the write passes hold more registers and staging.
+constexpr int csr_blocks_per_sm(int mode) { return mode == 0 ? 5 : 4; }
+constexpr int kAhead = 4;              // rows per lane whose offsets are loaded together
 constexpr int kScanBlock = 1024;
 constexpr int kScanItems = 4;
-constexpr int kScanGroup = kScanBlock * kScanItems;  // tiles per block of pass 3
+constexpr int kScanGroup = kScanBlock * kScanItems;  // segments per block of pass 3
 
-// tile_rows[t] = the row i with offsets[i] <= t * kCsrTile < offsets[i + 1].
-// Malformed offsets leave tiles unwritten; the conversion clamps what it reads.
-__global__ void __launch_bounds__(kBlock) csr_tile_rows_kernel(const int64_t *offsets, int32_t n, uint32_t ntiles,
-                                                               uint32_t *tile_rows)
+enum CsrMode : int { kCount = 0, kPairs, kRecords };
+
+// seg_rows[t] = the row i with offsets[i] <= t * kCsrSeg < offsets[i + 1].
+// A row of many segments is written by its whole warp.  Malformed offsets
+// leave segments unwritten; the conversion clamps what it reads.
+__global__ void __launch_bounds__(kBlock) csr_seg_rows_kernel(const int64_t *offsets, int32_t n, uint32_t nseg,
+                                                              uint32_t *seg_rows)
 {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const int64_t a = std::max<int64_t>(__ldg(offsets + i), 0), b = __ldg(offsets + i + 1);
-        if (a >= b)
-            continue;
-        const int64_t t1 = std::min<int64_t>((b - 1) / kCsrTile, (int64_t)ntiles - 1);
-        for (int64_t t = (a + kCsrTile - 1) / kCsrTile; t <= t1; t++)
-            tile_rows[t] = (uint32_t)i;
-    }
-}
-
-// The columns of this lane's kCsrItems entries of tile t (lane-striped).
-__device__ __forceinline__ void load_cols(const uint32_t *cols, int64_t nnz, uint32_t t, uint32_t ntiles,
-                                          uint32_t (&c)[kCsrItems])
-{
-    if (t >= ntiles)
-        return;
-    const int64_t j0 = (int64_t)t * kCsrTile + (threadIdx.x >> 5) * kCsrSeg + lane_id();
-#pragma unroll
-    for (int k = 0; k < kCsrItems; k++)
-        c[k] = j0 + 32 * k < nnz ? __ldcs(cols + j0 + 32 * k) : 0u;
-}
-
-// Thread 0: the row range of tile t into s_row[0..1] (the rows holding its
-// first and its last entry, clamped to [0, n)).
-__device__ __forceinline__ void load_row_range(const uint32_t *tile_rows, int32_t n, uint32_t t, uint32_t ntiles,
-                                               int32_t *s_row)
-{
-    if (t >= ntiles)
-        return;
-    const int32_t r0 = (int32_t)min(__ldg(tile_rows + t), (uint32_t)(n - 1));
-    const int32_t r1 = t + 1 < ntiles ? (int32_t)min(__ldg(tile_rows + t + 1), (uint32_t)(n - 1)) : n - 1;
-    s_row[0] = r0;
-    s_row[1] = max(r0, r1);
-}
-
-// Row marks of tile t: s_mark[o - first] = r for every non-empty row r that
-// starts inside the tile, and s_seg[w] = the row holding the first entry of
-// warp segment w when that row starts inside the tile (both stay 0 where the
-// row is row0).
-__device__ __forceinline__ void mark_rows(const int64_t *offsets, int64_t first, uint32_t len, int32_t row0,
-                                          int32_t row1, uint32_t *s_mark, uint32_t *s_seg)
-{
-    for (int64_t r = (int64_t)row0 + 1 + threadIdx.x; r <= row1; r += kCsrThreads) {
-        const int64_t o = __ldg(offsets + r);
-        if (o >= first + len)
-            break;
-        const int64_t on = __ldg(offsets + r + 1);
-        if (o > first && on > o) {
-            s_mark[o - first] = (uint32_t)r;
-            // warp segments whose first entry lies in [o, on)
-            const int64_t lo = (o - first + kCsrSeg - 1) / kCsrSeg, hi = (on - 1 - first) / kCsrSeg;
-            for (int64_t w = lo; w <= min(hi, (int64_t)kCsrWarps - 1); w++)
-                s_seg[w] = (uint32_t)r;
+    const uint32_t lane = lane_id();
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x; i0 < n; i0 += stride) {
+        const int64_t i = i0 + threadIdx.x;
+        int64_t t = 0, t1 = -1;
+        if (i < n) {
+            const int64_t a = std::max<int64_t>(__ldg(offsets + i), 0), b = __ldg(offsets + i + 1);
+            if (a < b) {
+                t = (a + kCsrSeg - 1) / kCsrSeg;
+                t1 = std::min<int64_t>((b - 1) / kCsrSeg, (int64_t)nseg - 1);
+            }
+        }
+        const bool wide = t1 - t >= 8;
+        if (!wide)
+            for (; t <= t1; t++)
+                seg_rows[t] = (uint32_t)i;
+        for (unsigned todo = __ballot_sync(0xffffffffu, wide); todo; todo &= todo - 1) {
+            const int src = __ffs(todo) - 1;
+            const int64_t from = __shfl_sync(0xffffffffu, t, src), to = __shfl_sync(0xffffffffu, t1, src);
+            const uint32_t row = (uint32_t)(i - (int64_t)lane + src);
+            for (int64_t q = from + lane; q <= to; q += 32)
+                seg_rows[q] = row;
         }
     }
 }
 
-// Rows of this lane's entries and their keep flags (bit k: entry k has
-// row < col), after mark_rows and a __syncthreads.  Each lane zeroes the
-// marks it reads (lane 0 its warp's segment row), so both are all zero again
-// once every warp has returned.  *kept: the warp's kept entries.
-__device__ __forceinline__ uint32_t resolve_rows(int64_t first, int64_t nnz, int32_t row0,
-                                                 const uint32_t (&col)[kCsrItems], uint32_t (&row)[kCsrItems],
-                                                 uint32_t *s_mark, uint32_t *s_seg, uint32_t *kept)
+// The columns of this lane's entries of segment t (zero past the end: below no
+// row).  `wide`: cols is 16-byte aligned.
+__device__ __forceinline__ void load_cols(const uint32_t *cols, int64_t nnz, uint32_t t, uint32_t nseg, bool wide,
+                                          uint32_t (&c)[kCsrItems])
 {
-    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    const uint32_t le = 0xffffffffu >> (31 - lane);  // lanes 0..lane
-    const int64_t j0 = first + warp * kCsrSeg + lane;
-    uint32_t *mk = s_mark + warp * kCsrSeg + lane;
-    uint32_t carry = max(s_seg[warp], (uint32_t)row0), keep = 0;
+    if (t >= nseg)
+        return;
+    const int64_t j0 = (int64_t)t * kCsrSeg + lane_id() * kCsrItems;
+    if (wide && j0 + kCsrItems <= nnz) {
+        const uint4 *p = reinterpret_cast<const uint4 *>(cols + j0);
+        const uint4 a = __ldcs(p), b = __ldcs(p + 1);
+        c[0] = a.x, c[1] = a.y, c[2] = a.z, c[3] = a.w;
+        c[4] = b.x, c[5] = b.y, c[6] = b.z, c[7] = b.w;
+        return;
+    }
+#pragma unroll
+    for (int k = 0; k < kCsrItems; k++)
+        c[k] = j0 + k < nnz ? __ldcs(cols + j0 + k) : 0u;
+}
+
+// The rows holding the first entry of segment t and of the next one, clamped
+// to [0, n).
+__device__ __forceinline__ void load_row_range(const uint32_t *seg_rows, int32_t n, uint32_t t, uint32_t nseg,
+                                               int32_t &row0, int32_t &row1)
+{
+    if (t >= nseg)
+        return;
+    row0 = (int32_t)min(__ldg(seg_rows + t), (uint32_t)(n - 1));
+    row1 = max(row0, t + 1 < nseg ? (int32_t)min(__ldg(seg_rows + t + 1), (uint32_t)(n - 1)) : n - 1);
+}
+
+// Rows of this lane's entries and their keep flags (bit k: entry k has
+// row < col).  mark[o - first] = r for every non-empty row r > row0 that starts
+// inside the segment.  Rows ascend, so an entry's row is the largest mark up to
+// it: a running maximum over the lane's eight marks and one scan over the
+// lanes.  Marks are never cleared: a warp's segments ascend, so what an earlier
+// one left is at most this one's row0.
+__device__ __forceinline__ uint32_t resolve_rows(const int64_t *offsets, int64_t first, int64_t end, int32_t row0,
+                                                 int32_t row1, uint32_t *mark, const uint32_t (&col)[kCsrItems],
+                                                 uint32_t (&row)[kCsrItems])
+{
+    const uint32_t lane = lane_id();
+    __syncwarp();  // the last segment's marks are read
+    {
+        const int64_t r = (int64_t)row0 + 1 + lane;
+        if (r <= row1) {
+            const int64_t o = __ldg(offsets + r), on = __ldg(offsets + r + 1);
+            if (o > first && o < end && on > o)
+                mark[o - first] = (uint32_t)r;
+        }
+    }
+    // a segment of nearly empty rows spans thousands of them: kAhead rows' loads
+    // per lane in flight together
+    for (int64_t r0 = (int64_t)row0 + 33 + lane; r0 <= row1; r0 += 32 * kAhead) {
+        int64_t o[kAhead], on[kAhead];
+#pragma unroll
+        for (int q = 0; q < kAhead; q++) {
+            const int64_t r = min(r0 + 32 * q, (int64_t)row1);
+            o[q] = __ldg(offsets + r);
+            on[q] = __ldg(offsets + r + 1);
+        }
+#pragma unroll
+        for (int q = 0; q < kAhead; q++)
+            if (r0 + 32 * q <= row1 && o[q] > first && o[q] < end && on[q] > o[q])
+                mark[o[q] - first] = (uint32_t)(r0 + 32 * q);
+    }
     __syncwarp();
+    const uint4 a = reinterpret_cast<const uint4 *>(mark)[2 * lane], b = reinterpret_cast<const uint4 *>(mark)[2 * lane + 1];
+    row[0] = max(a.x, (uint32_t)row0);
+    row[1] = max(row[0], a.y);
+    row[2] = max(row[1], a.z);
+    row[3] = max(row[2], a.w);
+    row[4] = max(row[3], b.x);
+    row[5] = max(row[4], b.y);
+    row[6] = max(row[5], b.z);
+    row[7] = max(row[6], b.w);
+    uint32_t before = row[7];  // the largest mark up to this lane's end ...
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, before, d);
+        if (lane >= (uint32_t)d)
+            before = max(before, y);
+    }
+    before = __shfl_up_sync(0xffffffffu, before, 1);  // ... up to the lane before
     if (lane == 0)
-        s_seg[warp] = 0;
+        before = (uint32_t)row0;
+    uint32_t keep = 0;
 #pragma unroll
     for (int k = 0; k < kCsrItems; k++) {
-        const uint32_t m = mk[32 * k];
-        mk[32 * k] = 0;
-        const uint32_t b = __ballot_sync(0xffffffffu, m != 0) & le;
-        const uint32_t v = __shfl_sync(0xffffffffu, m, b ? 31 - __clz(b) : 0);
-        row[k] = b ? v : carry;
-        carry = __shfl_sync(0xffffffffu, row[k], 31);
-        keep |= (uint32_t)(j0 + 32 * k < nnz && (int64_t)row[k] < (int64_t)col[k]) << k;
+        row[k] = max(row[k], before);
+        keep |= (uint32_t)(row[k] < col[k]) << k;
     }
-    uint32_t n_kept = __popc(keep);
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1)
-        n_kept += __shfl_xor_sync(0xffffffffu, n_kept, d);
-    *kept = n_kept;
     return keep;
 }
 
-// Pass 2: counts[t] += kept entries of tile t (counts zeroed beforehand).
-__global__ void __launch_bounds__(kCsrThreads, kCsrBlocksPerSm)
-    csr_count_kernel(const int64_t *offsets, const uint32_t *cols, int32_t n, int64_t nnz,
-                     const uint32_t *tile_rows, uint32_t *counts)
+// Passes 2 and 4.  kCount: counts[t] = kept entries of segment t.  kRecords:
+// {row, col, w[p]} to rec_out[p] for p < cap; kPairs: packed pairs to out.
+template <int MODE>
+__global__ void __launch_bounds__(kCsrThreads, csr_blocks_per_sm(MODE))
+    csr_pass_kernel(const int64_t *offsets, const uint32_t *cols, int32_t n, int64_t nnz, const uint32_t *seg_rows,
+                    uint32_t *counts, const uint32_t *prefix, const uint32_t *group_off, unsigned long long *out,
+                    const uint32_t *w, phem_edge *rec_out, uint64_t cap)
 {
-    __shared__ uint32_t s_mark[kCsrTile];
-    __shared__ uint32_t s_seg[kCsrWarps];
-    __shared__ int32_t s_row[2][2];
-    const uint32_t ntiles = (uint32_t)((nnz + kCsrTile - 1) / kCsrTile);
-    for (uint32_t i = threadIdx.x; i < kCsrTile; i += kCsrThreads)
-        s_mark[i] = 0;
-    if (threadIdx.x < kCsrWarps)
-        s_seg[threadIdx.x] = 0;
-    uint32_t t = blockIdx.x;
-    if (threadIdx.x == 0)
-        load_row_range(tile_rows, n, t, ntiles, s_row[0]);
+    __shared__ __align__(16) uint32_t s_mark[kCsrWarps][kCsrSeg];
+    __shared__ __align__(16) uint32_t s_out[kCsrWarps][MODE == kRecords ? kCsrSeg * 3 + 4 : 4];
+    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
+    const bool wide = ((uintptr_t)cols & 15) == 0;
+    const uint32_t nseg = (uint32_t)((nnz + kCsrSeg - 1) / kCsrSeg);
+    const uint32_t GW = gridDim.x * kCsrWarps;
+    uint32_t *mark = s_mark[warp];
+    for (uint32_t i = lane; i < kCsrSeg; i += 32)
+        mark[i] = 0;
+    uint32_t t = blockIdx.x * kCsrWarps + warp;
     uint32_t nc[kCsrItems];
-    load_cols(cols, nnz, t, ntiles, nc);
-    __syncthreads();
-    for (int buf = 0; t < ntiles; t += gridDim.x, buf ^= 1) {
-        uint32_t col[kCsrItems], row[kCsrItems], kept;
+    int32_t nrow0 = 0, nrow1 = 0;
+    load_row_range(seg_rows, n, t, nseg, nrow0, nrow1);
+    load_cols(cols, nnz, t, nseg, wide, nc);
+    for (; t < nseg; t += GW) {
+        uint32_t col[kCsrItems], row[kCsrItems];
 #pragma unroll
         for (int k = 0; k < kCsrItems; k++)
             col[k] = nc[k];
-        const int32_t row0 = s_row[buf][0], row1 = s_row[buf][1];
-        const uint32_t tn = t + gridDim.x;
-        if (threadIdx.x == 0)
-            load_row_range(tile_rows, n, tn, ntiles, s_row[buf ^ 1]);
-        load_cols(cols, nnz, tn, ntiles, nc);  // in flight while this tile resolves
-        const int64_t first = (int64_t)t * kCsrTile;
-        const uint32_t len = (uint32_t)min((int64_t)kCsrTile, nnz - first);
-        mark_rows(offsets, first, len, row0, row1, s_mark, s_seg);
-        __syncthreads();
-        resolve_rows(first, nnz, row0, col, row, s_mark, s_seg, &kept);
-        if (lane_id() == 0 && kept)
-            atomicAdd(counts + t, kept);
-        __syncthreads();  // marks read (and zeroed) before the next tile writes them
+        const int32_t row0 = nrow0, row1 = nrow1;
+        // in flight while this segment is worked on (no overflow: nseg < 2^24)
+        load_row_range(seg_rows, n, t + GW, nseg, nrow0, nrow1);
+        load_cols(cols, nnz, t + GW, nseg, wide, nc);
+        const uint64_t base = MODE == kCount ? 0 : (uint64_t)__ldg(prefix + t) + __ldg(group_off + t / kScanGroup);
+        const int64_t first = (int64_t)t * kCsrSeg;
+        const uint32_t keep = resolve_rows(offsets, first, min(first + kCsrSeg, nnz), row0, row1, mark, col, row);
+        if (MODE == kCount) {
+            const uint32_t kept = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(keep));
+            if (lane == 0)
+                counts[t] = kept;
+            continue;
+        }
+        uint32_t at = __popc(keep);  // place of the lane's first kept entry
+        const uint32_t own = at;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, at, d);
+            if (lane >= (uint32_t)d)
+                at += y;
+        }
+        uint32_t total = __shfl_sync(0xffffffffu, at, 31);
+        at -= own;
+        if (MODE == kPairs) {
+#pragma unroll
+            for (int k = 0; k < kCsrItems; k++)
+                if (keep >> k & 1)
+                    out[base + at++] = ((unsigned long long)row[k] << 32) | col[k];
+            continue;
+        }
+        if (base + total > cap)  // a wrong entry count: only the first cap records are written
+            total = base < cap ? (uint32_t)(cap - base) : 0u;
+        // at the output's own offset from a 16-byte boundary; the weights of
+        // the segment's records are contiguous
+        const uint32_t shift = (uint32_t)(base * 3) & 3u;
+        uint32_t *so = s_out[warp] + shift;
+        const uint32_t *wp = w + base;
+        for (uint32_t i = lane; i < total; i += 64) {
+            const uint32_t x = __ldcs(wp + i), y = i + 32 < total ? __ldcs(wp + i + 32) : 0u;
+            so[3 * i + 2] = x;
+            if (i + 32 < total)
+                so[3 * i + 98] = y;
+        }
+#pragma unroll
+        for (int k = 0; k < kCsrItems; k++)
+            if (keep >> k & 1) {
+                so[3 * at] = row[k];
+                so[3 * at + 1] = col[k];
+                at++;
+            }
+        __syncwarp();
+        const uint32_t end = shift + 3 * total;
+        uint32_t *g = reinterpret_cast<uint32_t *>(rec_out) + (base * 3 - shift);
+        for (uint32_t c = lane * 4; c < end; c += 128) {
+            const uint4 v = *reinterpret_cast<const uint4 *>(s_out[warp] + c);
+            if (c >= shift && c + 4 <= end) {
+                __stcs(reinterpret_cast<uint4 *>(g + c), v);
+            } else {
+                const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int x = 0; x < 4; x++)
+                    if (c + x >= shift && c + x < end)
+                        g[c + x] = q[x];
+            }
+        }
+        // (the next segment's resolve_rows synchronises before so is rewritten)
     }
 }
 
-// Pass 3: prefix[t] = kept entries before tile t within its group of
-// kScanGroup tiles (one block per group, kScanItems tiles per thread); the
+// Pass 3: prefix[t] = kept entries before segment t within its group of
+// kScanGroup (one block per group, kScanItems segments per thread); the
 // last block to finish scans the group totals into group_off[] and writes
 // the whole count to *kept.
-__global__ void __launch_bounds__(kScanBlock) csr_scan_kernel(const uint32_t *counts, uint32_t ntiles,
+__global__ void __launch_bounds__(kScanBlock) csr_scan_kernel(const uint32_t *counts, uint32_t nseg,
                                                               uint32_t *prefix, uint32_t *group_tot,
                                                               uint32_t *group_off, unsigned long long *kept,
                                                               unsigned long long *ticket)
@@ -226,14 +318,14 @@ __global__ void __launch_bounds__(kScanBlock) csr_scan_kernel(const uint32_t *co
     uint32_t v[kScanItems], sum = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        v[k] = i0 + k < ntiles ? counts[i0 + k] : 0u;
+        v[k] = i0 + k < nseg ? counts[i0 + k] : 0u;
         sum += v[k];
     }
     uint32_t total;
     uint32_t run = block_scan(sum, &total);
 #pragma unroll
     for (int k = 0; k < kScanItems; k++)
-        if (i0 + k < ntiles) {
+        if (i0 + k < nseg) {
             prefix[i0 + k] = run;
             run += v[k];
         }
@@ -262,85 +354,13 @@ __global__ void __launch_bounds__(kScanBlock) csr_scan_kernel(const uint32_t *co
         *kept = carry;
 }
 
-// Pass 4.  RECORDS: write {row, col, w[p]} to rec_out[p] for p < cap;
-// otherwise packed pairs to out.
-template <bool RECORDS>
-__global__ void __launch_bounds__(kCsrThreads, kCsrBlocksPerSm)
-    csr_write_kernel(const int64_t *offsets, const uint32_t *cols, int32_t n, int64_t nnz,
-                     const uint32_t *tile_rows, const uint32_t *prefix, const uint32_t *group_off,
-                     unsigned long long *out, const uint32_t *w, phem_edge *rec_out, uint64_t cap)
-{
-    __shared__ uint32_t s_mark[kCsrTile];
-    __shared__ uint32_t s_seg[kCsrWarps];
-    __shared__ uint32_t s_wsum[kCsrWarps];
-    __shared__ int32_t s_row[2][2];
-    const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    const uint32_t lt = (1u << lane) - 1u;  // lanes before this one
-    const uint32_t ntiles = (uint32_t)((nnz + kCsrTile - 1) / kCsrTile);
-    for (uint32_t i = threadIdx.x; i < kCsrTile; i += kCsrThreads)
-        s_mark[i] = 0;
-    if (threadIdx.x < kCsrWarps)
-        s_seg[threadIdx.x] = 0;
-    uint32_t t = blockIdx.x;
-    if (threadIdx.x == 0)
-        load_row_range(tile_rows, n, t, ntiles, s_row[0]);
-    uint32_t nc[kCsrItems];
-    load_cols(cols, nnz, t, ntiles, nc);
-    __syncthreads();
-    for (int buf = 0; t < ntiles; t += gridDim.x, buf ^= 1) {
-        uint32_t col[kCsrItems], row[kCsrItems], kept;
-#pragma unroll
-        for (int k = 0; k < kCsrItems; k++)
-            col[k] = nc[k];
-        const int32_t row0 = s_row[buf][0], row1 = s_row[buf][1];
-        const uint32_t base = __ldg(prefix + t) + __ldg(group_off + t / kScanGroup);
-        const uint32_t tn = t + gridDim.x;
-        if (threadIdx.x == 0)
-            load_row_range(tile_rows, n, tn, ntiles, s_row[buf ^ 1]);
-        load_cols(cols, nnz, tn, ntiles, nc);  // in flight while this tile resolves
-        const int64_t first = (int64_t)t * kCsrTile;
-        const uint32_t len = (uint32_t)min((int64_t)kCsrTile, nnz - first);
-        mark_rows(offsets, first, len, row0, row1, s_mark, s_seg);
-        __syncthreads();
-        const uint32_t keep = resolve_rows(first, nnz, row0, col, row, s_mark, s_seg, &kept);
-        if (lane == 0)
-            s_wsum[warp] = kept;
-        __syncthreads();  // also: every mark is read (and zeroed) before the next tile writes them
-        uint64_t pos = base;
-        for (uint32_t k = 0; k < warp; k++)
-            pos += s_wsum[k];
-#pragma unroll
-        for (int k = 0; k < kCsrItems; k++) {
-            const bool kp = keep >> k & 1;
-            const uint32_t b = __ballot_sync(0xffffffffu, kp);
-            if (kp) {
-                const uint64_t q = pos + __popc(b & lt);
-                if (RECORDS) {
-                    if (q < cap) {
-                        phem_edge rc;
-                        rc.u = row[k];
-                        rc.v = col[k];
-                        rc.w = __ldcs(w + q);
-                        rec_out[q] = rc;
-                    }
-                } else {
-                    out[q] = ((unsigned long long)row[k] << 32) | col[k];
-                }
-            }
-            pos += __popc(b);
-        }
-        // No barrier here: s_wsum is rewritten only after the next tile's
-        // first barrier, which every warp reaches after reading it.
-    }
-}
-
 }  // namespace
 
 size_t csr_scratch_bytes(int64_t nnz)
 {
-    const size_t tiles = (size_t)((nnz + kCsrTile - 1) / kCsrTile);
-    const size_t groups = (tiles + kScanGroup - 1) / kScanGroup;
-    return align256((3 * tiles + 1 + 2 * groups) * sizeof(uint32_t));
+    const size_t segs = (size_t)((nnz + kCsrSeg - 1) / kCsrSeg);
+    const size_t groups = (segs + kScanGroup - 1) / kScanGroup;
+    return align256((3 * segs + 1 + 2 * groups) * sizeof(uint32_t));
 }
 
 phem_status csr_launch_to_coo(phem_context *ctx, const int64_t *offsets, const uint32_t *cols, int32_t n,
@@ -351,39 +371,40 @@ phem_status csr_launch_to_coo(phem_context *ctx, const int64_t *offsets, const u
         set_error("csr: %lld entries (must be < 2^32)", (long long)nnz);
         return PHEM_ERR_INVALID;
     }
-    const uint64_t tiles = ((uint64_t)nnz + kCsrTile - 1) / kCsrTile;
-    if (tiles == 0 || n <= 0) {
+    const uint64_t segs = ((uint64_t)nnz + kCsrSeg - 1) / kCsrSeg;
+    if (segs == 0 || n <= 0) {
         PHEM_CUDA_TRY(cudaMemsetAsync(&ctx->ctl->misc[2], 0, sizeof(unsigned long long), ctx->stream));
         return PHEM_OK;
     }
-    const uint64_t groups = (tiles + kScanGroup - 1) / kScanGroup;
-    uint32_t *tile_rows = scratch, *counts = scratch + tiles + 1, *prefix = counts + tiles;
-    uint32_t *group_tot = prefix + tiles, *group_off = group_tot + groups;
-    const int blocks = (int)std::min<uint64_t>(tiles, (uint64_t)ctx->sm_count * kCsrBlocksPerSm);
+    const uint64_t groups = (segs + kScanGroup - 1) / kScanGroup;
+    uint32_t *seg_rows = scratch, *counts = scratch + segs + 1, *prefix = counts + segs;
+    uint32_t *group_tot = prefix + segs, *group_off = group_tot + groups;
+    auto *o = reinterpret_cast<unsigned long long *>(out);
+    auto pass = [&](auto kernel, int mode) {
+        KernelScope k(ctx, kKCsrCoo);
+        const int blocks = (int)std::min<uint64_t>((segs + kCsrWarps - 1) / kCsrWarps,
+                                                   (uint64_t)ctx->sm_count * csr_blocks_per_sm(mode));
+        kernel<<<blocks, kCsrThreads, 0, ctx->stream>>>(offsets, cols, n, nnz, seg_rows, counts, prefix, group_off, o, w,
+                                                        records, cap);
+    };
     {
         KernelScope k(ctx, kKCsrCoo);
         const int rblocks = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n + kBlock - 1) / kBlock,
                                                                          (int64_t)ctx->sm_count * 8));
-        csr_tile_rows_kernel<<<rblocks, kBlock, 0, ctx->stream>>>(offsets, n, (uint32_t)tiles, tile_rows);
+        csr_seg_rows_kernel<<<rblocks, kBlock, 0, ctx->stream>>>(offsets, n, (uint32_t)segs, seg_rows);
     }
-    PHEM_CUDA_TRY(cudaMemsetAsync(counts, 0, tiles * sizeof(uint32_t), ctx->stream));
-    {
-        KernelScope k(ctx, kKCsrCoo);
-        csr_count_kernel<<<blocks, kCsrThreads, 0, ctx->stream>>>(offsets, cols, n, nnz, tile_rows, counts);
-    }
+    pass(csr_pass_kernel<kCount>, kCount);
     PHEM_CUDA_TRY(cudaMemsetAsync(&ctx->ctl->misc[3], 0, sizeof(unsigned long long), ctx->stream));  // scan ticket
     {
         KernelScope k(ctx, kKCsrCoo);
-        csr_scan_kernel<<<(unsigned)groups, kScanBlock, 0, ctx->stream>>>(counts, (uint32_t)tiles, prefix, group_tot,
+        csr_scan_kernel<<<(unsigned)groups, kScanBlock, 0, ctx->stream>>>(counts, (uint32_t)segs, prefix, group_tot,
                                                                          group_off, &ctx->ctl->misc[2],
                                                                          &ctx->ctl->misc[3]);
     }
-    if (records || out) {
-        KernelScope k(ctx, kKCsrCoo);
-        auto *o = reinterpret_cast<unsigned long long *>(out);
-        (records ? csr_write_kernel<true> : csr_write_kernel<false>)<<<blocks, kCsrThreads, 0, ctx->stream>>>(
-            offsets, cols, n, nnz, tile_rows, prefix, group_off, o, w, records, cap);
-    }
+    if (records)
+        pass(csr_pass_kernel<kRecords>, kRecords);
+    else if (out)
+        pass(csr_pass_kernel<kPairs>, kPairs);
     PHEM_CUDA_TRY(cudaGetLastError());
     return PHEM_OK;
 }

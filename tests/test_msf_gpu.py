@@ -380,3 +380,39 @@ def test_one_cta_solve_sizes(ctx, n, m):
     f = P.api.forest_set(rd.forest)
     assert rd.components == rc.components == n - len(f) == n - rd.forest_edges
     np.testing.assert_array_equal(oracle.cc_solve(f, n)[0], labels)
+
+
+@pytest.mark.parametrize("kind", ["segments", "long_empty_runs"])
+@pytest.mark.parametrize("skew", [0, 1, 3])
+def test_csr_segments(ctx, kind, skew):
+    """Rows that start and end at and around the 256-entry segments, segments
+    that span thousands of empty rows, and a column array at every 4-byte
+    alignment, as pairs and as records (16-byte stores at every offset)."""
+    import torch
+    rng = np.random.default_rng(5)
+    if kind == "segments":
+        lens = np.array([256, 255, 257, 1, 512, 0, 31, 33, 32, 7, 9, 768, 2, 2047, 2049, 0, 5], np.int64)
+        n = 6000
+        rows = np.repeat(np.arange(len(lens)), lens)
+    else:
+        n = 400000
+        rows = np.sort(np.r_[rng.integers(0, 200, 1000), rng.integers(200, n - 1, 3000), np.full(300, n - 2)])
+    cols = rng.integers(0, n, len(rows))
+    off, cols = _csr_from_entries(rows, cols, n)
+    want = oracle.csr_to_coo(off, cols, n)
+    d_off = torch.from_numpy(off).cuda()
+    d_cols = torch.from_numpy(np.concatenate([np.zeros(skew, np.uint32), cols]).view(np.int32)).cuda()[skew:]
+    d_out = torch.empty(len(cols), dtype=torch.int64, device="cuda")
+    k = _lib.C.c_int64()
+    torch.cuda.synchronize()
+    _lib.check(_lib.lib().phem_csr_to_coo(ctx._h, d_off.data_ptr(), d_cols.data_ptr(), n, d_out.data_ptr(),
+                                          _lib.C.byref(k)), "phem_csr_to_coo")
+    assert k.value == len(want)
+    np.testing.assert_array_equal(d_out[: k.value].cpu().numpy().view(np.uint64), want)
+    w = rng.integers(1, 1 << 20, len(want)).astype(np.uint32)
+    E = np.zeros((len(want), 3), np.uint32)
+    E[:, 0], E[:, 1], E[:, 2] = want >> np.uint64(32), want & np.uint64(0xFFFFFFFF), w
+    ids, cnt, tot = expect(E, n)
+    d_w = torch.from_numpy(w.view(np.int32)).cuda()
+    torch.cuda.synchronize()
+    assert_msf(ctx.msf_solve_csr(d_off, d_cols, n, d_w, len(want)), E, ids, cnt, tot)
