@@ -23,7 +23,7 @@ thread_local char g_last_error[512] = "";
 
 const char *const kKernelNames[kKernelCount] = {
     "cc_solve", "msf_solve", "msf_init", "msf_select", "msf_edge_pass", "msf_hook", "msf_compress", "msf_gather",
-    "cc_init", "cc_unite", "cc_merge", "cc_label", "cc_minid", "cc_count", "csr_to_coo", "batch_solve"};
+    "cc_init", "cc_unite", "cc_merge", "cc_label", "cc_count", "csr_to_coo", "batch_solve"};
 
 constexpr size_t kLaunchLogCap = 1u << 16;
 
@@ -300,8 +300,11 @@ phem_status phem_context_create(int device, phem_context **out)
     c->stream = c->own_stream;
     if (cudaMalloc(&c->ctl, sizeof(Ctl)) != cudaSuccess)
         return fail("control block");
-    if (cudaMallocHost(&c->h_ctl, sizeof(Ctl)) != cudaSuccess)
+    if (cudaMalloc(&c->solve_ctl, sizeof(Ctl)) != cudaSuccess)
+        return fail("solve control block");
+    if (cudaMallocHost(&c->h_ctl, sizeof(Ctl) + sizeof(uint64_t)) != cudaSuccess)
         return fail("pinned control block");
+    c->h_kept = reinterpret_cast<uint64_t *>(c->h_ctl + 1);
     if (cudaEventCreate(&c->ev_start) != cudaSuccess || cudaEventCreate(&c->ev_stop) != cudaSuccess)
         return fail("events");
     if (cudaMemset(c->ctl, 0, sizeof(Ctl)) != cudaSuccess)
@@ -325,6 +328,8 @@ void phem_context_destroy(phem_context *ctx)
         cudaFree(ctx->status);
     if (ctx->ctl)
         cudaFree(ctx->ctl);
+    if (ctx->solve_ctl)
+        cudaFree(ctx->solve_ctl);
     if (ctx->h_ctl)
         cudaFreeHost(ctx->h_ctl);
     if (ctx->tiny_host)
@@ -690,13 +695,13 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
     if (canonical) {
         plan.e0 = d_edges;
         plan.forest = d_for;
+        plan.label = d_lab;
         PHEM_TRY(msf_run(ctx, kKindPacked, plan));
-        // plan.best is free after the rounds: reuse it as the per-root min-id array
-        PHEM_TRY(cc_launch_minid_labels(ctx, n, plan.parent, reinterpret_cast<uint32_t *>(plan.best), d_lab));
     } else if (one_launch) {
         PHEM_TRY(cc_grid(ctx, d_edges, m, s, n, d_lab, d_for, static_cast<char *>(ctx->ws) + base + o_par));
     } else {
         int32_t *d_par = reinterpret_cast<int32_t *>(static_cast<char *>(ctx->ws) + base + o_par);
+        ctx->publishes = false;
         PHEM_CUDA_TRY(cudaMemsetAsync(ctx->ctl, 0, sizeof(Ctl), ctx->stream));
         PHEM_TRY(cc_launch_init(ctx, n, d_par, nullptr, d_for));
         if (overlap) {
@@ -711,7 +716,8 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
         PHEM_TRY(cc_launch_label(ctx, n, d_par, d_lab));
     }
     cudaEventRecord(ctx->ev_stop, ctx->stream);
-    if (!one_launch)
+    const bool counted = canonical || one_launch;
+    if (!counted)
         PHEM_TRY(cc_launch_count(ctx, n, d_lab, d_for));
     PHEM_TRY(copy_back(ctx, sl, lb));
     PHEM_TRY(copy_back(ctx, sf, fb));
@@ -722,7 +728,7 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
     if (stats) {
         stats->components = (uint32_t)ctx->h_ctl->misc[0];
         stats->forest_edges =
-            d_for && !one_launch ? ctx->h_ctl->misc[1] : (uint64_t)n - ctx->h_ctl->misc[0];
+            d_for && !counted ? ctx->h_ctl->misc[1] : (uint64_t)n - ctx->h_ctl->misc[0];
         stats->rounds = rounds;
         stats->device_ms = ms;
     }
@@ -1050,8 +1056,8 @@ static phem_status msf_common(phem_context *ctx, const phem_edge *edges, uint64_
     PHEM_TRY(msf_run(ctx, kKindMsf, plan));
     PHEM_CUDA_TRY(cudaEventRecord(ctx->ev_stop, ctx->stream));
     if (d_count_total)
-        PHEM_CUDA_TRY(cudaMemcpyAsync(d_count_total, &ctx->ctl->msf_count, 2 * sizeof(uint64_t),
-                                      cudaMemcpyDeviceToDevice, ctx->stream));
+        PHEM_CUDA_TRY(cudaMemcpyAsync(d_count_total, &(ctx->publishes ? ctx->h_ctl : ctx->ctl)->msf_count,
+                                      2 * sizeof(uint64_t), cudaMemcpyDefault, ctx->stream));
     PHEM_TRY(msf_finish(ctx, &rounds, "msf"));
     const Ctl &h = *ctx->h_ctl;
     if (h.msf_count > (uint64_t)n - 1 + (n == 0)) {
@@ -1273,7 +1279,7 @@ phem_status phem_msf_solve_csr(phem_context *ctx, const int64_t *offsets, const 
                  rb = (size_t)m_upper * sizeof(phem_edge);
     const size_t o_off = 0, o_col = align256(ob), o_w = o_col + align256(cb), o_tr = o_w + align256(wb),
                  o_rec = o_tr + tb;
-    PHEM_TRY(input_reserve(ctx, o_rec + align256(rb) + 256));
+    PHEM_TRY(input_reserve(ctx, o_rec + align256(rb)));
     char *b = static_cast<char *>(ctx->input);
     auto put = [&](const void *src, size_t bytes, size_t off) -> const void * {
         if (is_device_ptr(src))
@@ -1288,26 +1294,17 @@ phem_status phem_msf_solve_csr(phem_context *ctx, const int64_t *offsets, const 
     uint32_t *d_tr = reinterpret_cast<uint32_t *>(b + o_tr);
     phem_edge *d_rec = reinterpret_cast<phem_edge *>(b + o_rec);
     // one pass: kept entry p becomes the record {row, col, weights[p]}
-    phem_status st = csr_launch_to_coo(ctx, d_off, d_col, (int32_t)n, nnz, d_tr, nullptr, d_w, d_rec, m_upper);
+    PHEM_TRY(csr_launch_to_coo(ctx, d_off, d_col, (int32_t)n, nnz, d_tr, nullptr, d_w, d_rec, m_upper));
     // The solve is queued behind the conversion with no host round trip
-    // between them; the conversion's count of entries with row < col is kept
-    // aside (the solve resets the control block) and checked afterwards.  The
-    // conversion writes no record past m_upper, and a short count leaves stale
-    // records that the solve range-checks like any input, so a mismatch only
-    // discards the solve's result.
-    uint64_t *d_kept = reinterpret_cast<uint64_t *>(b + o_rec + align256(rb));
-    if (st == PHEM_OK && cudaMemcpyAsync(d_kept, &ctx->ctl->misc[2], sizeof(uint64_t), cudaMemcpyDeviceToDevice,
-                                         ctx->stream) != cudaSuccess)
-        st = PHEM_ERR_CUDA;
-    if (st != PHEM_OK)
-        return st;
+    // between them; the conversion writes its count of entries with row < col
+    // to pinned host memory, where it is checked afterwards.  The conversion
+    // writes no record past m_upper, and a short count leaves stale records
+    // that the solve range-checks like any input, so a mismatch only discards
+    // the solve's result.
     const phem_status solved = msf_common(ctx, d_rec, m_upper, n, msf, count, total, stats, nullptr);
-    uint64_t kept = 0;
-    if (cudaMemcpyAsync(&ctx->h_ctl->misc[2], d_kept, sizeof(uint64_t), cudaMemcpyDeviceToHost, ctx->stream) !=
-        cudaSuccess)
-        return PHEM_ERR_CUDA;
-    PHEM_TRY(stream_wait(ctx));
-    kept = ctx->h_ctl->misc[2];
+    if (solved != PHEM_OK)  // it may have ended before it waited
+        PHEM_TRY(stream_wait(ctx));
+    const uint64_t kept = *ctx->h_kept;
     if (kept != m_upper) {
         set_error("msf_solve_csr: CSR has %llu entries with row < col, m_upper = %llu",
                   (unsigned long long)kept, (unsigned long long)m_upper);

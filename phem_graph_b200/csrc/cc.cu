@@ -105,44 +105,6 @@ __global__ void __launch_bounds__(kBlock) cc_compress_kernel(int32_t n, int32_t 
     }
 }
 
-__device__ __forceinline__ uint32_t plain_root(const uint32_t *parent, uint32_t x, uint32_t n, uint32_t *err)
-{
-    for (uint32_t steps = 0; steps <= n; steps++) {
-        const uint32_t p = parent[x];
-        if (p == x)
-            return x;
-        x = p;
-    }
-    set_err(err, kErrChase);
-    return x;
-}
-
-__global__ void __launch_bounds__(kBlock) minid_scatter_kernel(int32_t n, const uint32_t *parent, uint32_t *minid,
-                                                               uint32_t *err)
-{
-    // Lanes of a warp hold consecutive vertices, so among the lanes that share
-    // a root the lowest lane has the smallest id: only it reads the guard
-    // (through L1: a stale value is never below the true minimum) and
-    // offers.  A giant component's vertices no longer all hit one word.
-    const int32_t stride = gridDim.x * blockDim.x;
-    for (int32_t i0 = blockIdx.x * blockDim.x; i0 < n; i0 += stride) {
-        const int32_t i = i0 + (int32_t)threadIdx.x;
-        const bool in = i < n;
-        const uint32_t r = in ? plain_root(parent, (uint32_t)i, (uint32_t)n, err) : 0xffffffffu;
-        const unsigned peers = __match_any_sync(0xffffffffu, r);
-        if (in && (int)lane_id() == __ffs(peers) - 1 && (uint32_t)i < __ldca(minid + r))
-            atomicMin(minid + r, (uint32_t)i);
-    }
-}
-
-__global__ void __launch_bounds__(kBlock) minid_label_kernel(int32_t n, const uint32_t *parent,
-                                                             const uint32_t *minid, int32_t *label, uint32_t *err)
-{
-    const int32_t stride = gridDim.x * blockDim.x;
-    for (int32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        label[i] = (int32_t)minid[plain_root(parent, (uint32_t)i, (uint32_t)n, err)];
-}
-
 // Counts roots (label[i] == i) and filled forest slots into ctl->misc[0..1].
 __global__ void __launch_bounds__(kBlock) cc_count_kernel(int32_t n, const int32_t *label,
                                                           const unsigned long long *forest, Ctl *ctl)
@@ -233,22 +195,6 @@ phem_status cc_launch_merge(phem_context *ctx, const uint64_t *fa, const uint64_
     cc_merge_kernel<<<grid_for(ctx, fb ? 2 * (int64_t)n : n, 8), kBlock, 0, ctx->stream>>>(
         reinterpret_cast<const unsigned long long *>(fa), reinterpret_cast<const unsigned long long *>(fb), n,
         parent, reinterpret_cast<unsigned long long *>(forest_out), &ctx->ctl->err);
-    PHEM_CUDA_TRY(cudaGetLastError());
-    return PHEM_OK;
-}
-
-phem_status cc_launch_minid_labels(phem_context *ctx, int32_t n, uint32_t *parent, uint32_t *minid, int32_t *label)
-{
-    PHEM_CUDA_TRY(cudaMemsetAsync(minid, 0xff, sizeof(uint32_t) * (size_t)n, ctx->stream));
-    const int g = grid_for(ctx, n, 8);
-    {
-        KernelScope k(ctx, kKMinid);
-        minid_scatter_kernel<<<g, kBlock, 0, ctx->stream>>>(n, parent, minid, &ctx->ctl->err);
-    }
-    {
-        KernelScope k(ctx, kKMinid);
-        minid_label_kernel<<<g, kBlock, 0, ctx->stream>>>(n, parent, minid, label, &ctx->ctl->err);
-    }
     PHEM_CUDA_TRY(cudaGetLastError());
     return PHEM_OK;
 }

@@ -53,6 +53,7 @@ struct CcArgs {
     uint32_t *hooked;
     uint64_t seg;
     Ctl *ctl;
+    Ctl *publish;            // pinned host copy of the results, for the last kernel
     int timing;              // record phase timestamps
 };
 
@@ -390,6 +391,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) cc_grid_kernel(const __grid_
     full_compress(a.parent, a.n, nullptr, nullptr, 0, false, &ctl->err);
     count_roots(a, &s.acc);
     clock.stamp(kKCcLabel);
+    publish_ctl(ctl, a.publish);
 }
 
 // The edges behind the prefix.  A lane takes four consecutive edges of a
@@ -482,6 +484,7 @@ __global__ void __launch_bounds__(kBlock) cc_label_count_kernel(const __grid_con
     __syncthreads();
     full_compress(a.parent, a.n, nullptr, nullptr, 0, false, &a.ctl->err);
     count_roots(a, &s_roots);
+    publish_ctl(a.ctl, a.publish);
 }
 
 }  // namespace
@@ -510,9 +513,8 @@ phem_status cc_grid(phem_context *ctx, const uint64_t *d_edges, int64_t m, int64
     a.list = reinterpret_cast<uint4 *>(base + c.take<uint4>(a.seg * warps));
     a.hooked = reinterpret_cast<uint32_t *>(base + c.take<uint32_t>(a.seg * warps));
     a.giant = reinterpret_cast<uint32_t *>(base + c.take<uint32_t>(((uint64_t)n + 31) / 32));
-    a.ctl = ctx->ctl;
     a.timing = ctx->profiling;
-    PHEM_CUDA_TRY(cudaMemsetAsync(ctx->ctl, 0, sizeof(Ctl), ctx->stream));
+    PHEM_TRY(solve_ctl(ctx, &a.ctl, &a.publish));
     void *params[] = {&a};
     {
         KernelScope ks(ctx, kKCcSolve);

@@ -28,14 +28,14 @@ constexpr uint32_t kUnionRetryCap = 1u << 16;  // CAS retries per union
 constexpr uint32_t kLookbackSpinCap = 1u << 20; // waits per look-back window (~1 s)
 
 // ---------------------------------------------------------------- device control block
-// Small per-context device structure, zeroed at the start of each solve.
+// Small per-context device structure, zero at the start of each solve.
 constexpr uint32_t kMaxBarriers = 3 * PHEM_MAX_ROUNDS + 8;  // grid barriers of one MSF solve
 constexpr uint32_t kMaxPhases = kMaxBarriers + 8;
 struct Ctl {
     uint32_t err;
     uint32_t round;                                  // Boruvka rounds run
     uint32_t light_rounds;                           // rounds spent in the light phase
-    uint32_t ticket;                                 // tile tickets (R-MAT generator)
+    uint32_t ticket;                                 // tile tickets (R-MAT generator), CTAs done (publish_ctl)
     unsigned long long threshold;                    // light edge <=> key < threshold
     unsigned long long m_r[PHEM_MAX_ROUNDS + 1];     // live edges entering round r (exact)
     unsigned long long n_r[PHEM_MAX_ROUNDS + 1];     // components with a live edge in round r
@@ -43,12 +43,14 @@ struct Ctl {
     unsigned long long msf_total;
     unsigned long long misc[8];
     // from here on only the device (and profiling) looks
-    unsigned long long bar[kMaxBarriers];            // one word per grid barrier of the MSF solve
+    unsigned long long bar[kMaxBarriers];            // one word per grid barrier of a solve
     unsigned long long stamp[kMaxPhases];            // profiling: end time of each phase (ns)
     uint32_t phase_of[kMaxPhases];                   // ... and the phase's name (KernelId)
     uint32_t stamps;
     uint32_t pad0;
 };
+
+constexpr uint32_t kCtlPending = 0xffffffffu;  // host copy's err until a solve publishes its results
 
 // Input of an edge pass.
 enum : uint32_t {

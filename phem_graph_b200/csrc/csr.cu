@@ -274,10 +274,11 @@ __global__ void __launch_bounds__(kCsrThreads, csr_blocks_per_sm(MODE))
 // Pass 3: prefix[t] = kept entries before segment t within its group of
 // kScanGroup (one block per group, kScanItems segments per thread); the
 // last block to finish scans the group totals into group_off[] and writes
-// the whole count to *kept.
+// the whole count to *kept and to the host's pinned *host_kept.
 __global__ void __launch_bounds__(kScanBlock) csr_scan_kernel(const uint32_t *counts, uint32_t nseg,
                                                               uint32_t *prefix, uint32_t *group_tot,
                                                               uint32_t *group_off, unsigned long long *kept,
+                                                              unsigned long long *host_kept,
                                                               unsigned long long *ticket)
 {
     __shared__ uint32_t s_w[kScanBlock / 32 + 1];
@@ -351,7 +352,7 @@ __global__ void __launch_bounds__(kScanBlock) csr_scan_kernel(const uint32_t *co
         carry += s;
     }
     if (threadIdx.x == 0)
-        *kept = carry;
+        *kept = *host_kept = carry;
 }
 
 }  // namespace
@@ -374,6 +375,7 @@ phem_status csr_launch_to_coo(phem_context *ctx, const int64_t *offsets, const u
     const uint64_t segs = ((uint64_t)nnz + kCsrSeg - 1) / kCsrSeg;
     if (segs == 0 || n <= 0) {
         PHEM_CUDA_TRY(cudaMemsetAsync(&ctx->ctl->misc[2], 0, sizeof(unsigned long long), ctx->stream));
+        *ctx->h_kept = 0;
         return PHEM_OK;
     }
     const uint64_t groups = (segs + kScanGroup - 1) / kScanGroup;
@@ -399,6 +401,7 @@ phem_status csr_launch_to_coo(phem_context *ctx, const int64_t *offsets, const u
         KernelScope k(ctx, kKCsrCoo);
         csr_scan_kernel<<<(unsigned)groups, kScanBlock, 0, ctx->stream>>>(counts, (uint32_t)segs, prefix, group_tot,
                                                                          group_off, &ctx->ctl->misc[2],
+                                                                         reinterpret_cast<unsigned long long *>(ctx->h_kept),
                                                                          &ctx->ctl->misc[3]);
     }
     if (records)

@@ -17,7 +17,7 @@ enum KernelId : int {
     kKCcSolve = 0,  // the one-launch CC solve; phases: kKCcInit, kKCcUnite, kKCcLabel
     kKSolve,        // the MSF solve; the next six are its phases (device timestamps, no launches)
     kKInit, kKSelect, kKEdgePass, kKHook, kKCompress, kKGather,
-    kKCcInit, kKCcUnite, kKCcMerge, kKCcLabel, kKMinid, kKCcCount, kKCsrCoo, kKBatch,
+    kKCcInit, kKCcUnite, kKCcMerge, kKCcLabel, kKCcCount, kKCsrCoo, kKBatch,
     kKernelCount
 };
 extern const char *const kKernelNames[kKernelCount];
@@ -55,6 +55,10 @@ struct phem_context {
     size_t status_words = 0;           // (zeroed when grown; epochs keep old words from matching)
     phem::Ctl *ctl = nullptr;          // device control block
     phem::Ctl *h_ctl = nullptr;        // pinned host mirror of the control block
+    uint64_t *h_kept = nullptr;        // pinned, behind h_ctl: the CSR conversion's count
+    phem::Ctl *solve_ctl = nullptr;    // control block of solves that publish their results themselves
+    bool solve_ctl_zero = false;       // ... the last one zeroed it
+    bool publishes = false;            // the queued solve does
     void *tiny_host = nullptr;         // pinned staging of small host solves (tiny.cu), made on first use
     uint32_t tiny_ready = 0;           // bit k: launch attributes of small-solve kernel k are set
     uint64_t epoch = 1;                // look-back epoch counter
@@ -260,6 +264,7 @@ struct MsfPlan {
     uint4 *list;             // survivor segments, one per warp
     uint32_t *hooked;        // hooked-root segments, one per warp
     uint64_t *forest;        // kKindPacked only: forest slot per hooked root (may be null)
+    int32_t *label;          // kKindPacked only: min-id labels, components in misc[0] (may be null)
     phem_edge *out;          // kKindMsf with gather: the ordered MSF records (may be null)
     int gather;              // kKindMsf: rank and write the MSF records, count and total
 };
@@ -271,8 +276,12 @@ phem_status msf_plan(phem_context *ctx, const void *d_e0, uint64_t m, uint32_t n
                      size_t *extra_off);
 // Queues the whole solve (one launch); msf_finish waits and checks.
 phem_status msf_run(phem_context *ctx, int kind, MsfPlan &plan);
-// Waits for the queued work and checks it (copies the control block's results
-// to ctx->h_ctl).
+// The control block of the solve about to be queued, zero when its kernels
+// start, and where its last kernel publishes the results (null: msf_finish
+// copies them).
+phem_status solve_ctl(phem_context *ctx, Ctl **ctl, Ctl **publish);
+// Waits for the queued work and checks it; the control block's results are
+// then in ctx->h_ctl.
 phem_status msf_finish(phem_context *ctx, uint32_t *rounds_out, const char *what);
 
 // ---- CC engine (cc.cu) ----
@@ -284,9 +293,6 @@ phem_status cc_launch_label(phem_context *ctx, int32_t n, int32_t *parent, int32
 phem_status cc_launch_compress(phem_context *ctx, int32_t n, int32_t *parent);
 phem_status cc_launch_merge(phem_context *ctx, const uint64_t *fa, const uint64_t *fb, int32_t n, int32_t *parent,
                             uint64_t *forest_out);
-// min-id labels from an arbitrary-root parent array (canonical forest path)
-phem_status cc_launch_minid_labels(phem_context *ctx, int32_t n, uint32_t *parent, uint32_t *minid,
-                                   int32_t *label);
 phem_status cc_launch_count(phem_context *ctx, int32_t n, const int32_t *label, const uint64_t *forest);
 
 // ---- CC in one launch (cc_grid.cu) ----
@@ -299,7 +305,7 @@ SolveGrid cc_grid_size(int64_t m, int sm_count);
 size_t cc_grid_bytes(int64_t m, int64_t s, int32_t n, int sm_count);
 // Queues the whole solve over device edges (16-byte aligned; s a multiple of
 // four unless s = m): labels, forest slots (may be null), and the number of
-// components in ctx->ctl->misc[0].
+// components in misc[0] of the results (msf_finish).
 phem_status cc_grid(phem_context *ctx, const uint64_t *d_edges, int64_t m, int64_t s, int32_t n, int32_t *d_labels,
                     uint64_t *d_forest, void *ws);
 
@@ -308,7 +314,7 @@ phem_status cc_grid(phem_context *ctx, const uint64_t *d_edges, int64_t m, int64
 // and offsets).
 size_t csr_scratch_bytes(int64_t nnz);
 // Queues the conversion of a device CSR with nnz entries; the kept count lands
-// in ctx->ctl->misc[2].  With records set, the kept entry at position p is
+// in ctx->ctl->misc[2] and *ctx->h_kept.  With records set, the kept entry at position p is
 // written as {row, col, w[p]} to records[p] for p < cap (out is ignored);
 // otherwise packed pairs go to out, or only the count when out is null.
 phem_status csr_launch_to_coo(phem_context *ctx, const int64_t *offsets, const uint32_t *cols, int32_t n,

@@ -438,6 +438,42 @@ __device__ __forceinline__ void gather_pass(const SolveArgs &a, SolveSmem &s, ui
     }
 }
 
+// ---- min-id labels (packed edges) ----------------------------------------------
+//
+// Every vertex to its root, and the smallest id of each component to its
+// root's label, which the other vertices then copy.  Lanes hold consecutive
+// vertices, so of the lanes that share a root the lowest has the smallest id:
+// only it reads the guard (through L1: a stale value is never below the true
+// minimum) and offers.  2^20 vertices, 2^23 edges, us per call: as four launches
+// behind the solve 528, here 514 (inlined, with more spills, 532).
+__device__ __noinline__ void min_ids(const SolveArgs &a, SolveSmem &s)
+{
+    full_compress(a.parent, a.n, nullptr, nullptr, 0, false, &a.ctl->err);
+    uint32_t *mins = reinterpret_cast<uint32_t *>(a.label);
+    uint32_t roots = 0;
+    // full_compress's own vertices, whose roots this thread wrote
+    const uint64_t step = (uint64_t)gridDim.x * blockDim.x * kVItems;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x * kVItems; i0 < a.n; i0 += step) {
+        uint32_t r[kVItems], seen[kVItems];
+#pragma unroll
+        for (int k = 0; k < kVItems; k++) {
+            const uint64_t i = i0 + k * blockDim.x + threadIdx.x;
+            r[k] = i < a.n ? a.parent[i] : 0xffffffffu;
+            roots += i < a.n && r[k] == i;
+            const unsigned peers = __match_any_sync(0xffffffffu, r[k]);
+            const bool first = i < a.n && (int)lane_id() == __ffs(peers) - 1;
+            seen[k] = first ? __ldca(mins + r[k]) : 0u;
+        }
+#pragma unroll
+        for (int k = 0; k < kVItems; k++) {
+            const uint32_t i = (uint32_t)(i0 + k * blockDim.x + threadIdx.x);
+            if (i < seen[k])
+                atomicMin(mins + r[k], i);
+        }
+    }
+    acc_add(s, roots);
+}
+
 // ---- the solve ---------------------------------------------------------------
 
 template <int KIND>
@@ -463,6 +499,8 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(const __grid_co
             a.best[x] = kKeyNone;
             if (KIND == kKindPacked && a.forest)
                 a.forest[x] = kForestEmpty;
+            if (KIND == kKindPacked && a.label)
+                a.label[x] = -1;  // the largest unsigned id
         }
         if (KIND == kKindMsf) {
             const uint64_t words = (a.m + 31) / 32;
@@ -577,6 +615,21 @@ __global__ void __launch_bounds__(kSolveThreads, 1) solve_kernel(const __grid_co
         gather_pass(a, s, per);
         clock.stamp(kKGather);
     }
+    if (KIND == kKindPacked && a.label) {
+        min_ids(a, s);
+        if (!grid_sync(ctl, s, seq))
+            return;
+        if (lead)
+            ctl->misc[0] = s.sum;  // components
+        const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
+        for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + tid; x < a.n; x += step) {
+            const uint32_t root = __ldcg(a.parent + x);
+            if (root != x)
+                a.label[x] = __ldcg(a.label + root);
+        }
+        clock.stamp(kKCcLabel);
+    }
+    publish_ctl(ctl, a.publish);
 }
 
 // Light/heavy split: about lpv * n light edges, and only when the input is at
@@ -660,7 +713,7 @@ phem_status run_impl(phem_context *ctx, MsfPlan &plan)
     a.forest = reinterpret_cast<unsigned long long *>(plan.forest);
     a.out = plan.out;
     a.gather = plan.gather;
-    a.ctl = ctx->ctl;
+    a.label = plan.label;
     a.timing = ctx->profiling;
     // packed edges: the first k by index are light; the canonical forest's
     // slots follow from the rounds, so this rule is the same at every size
@@ -677,7 +730,7 @@ phem_status run_impl(phem_context *ctx, MsfPlan &plan)
     constexpr uint32_t rec_bytes = KIND == kKindMsf ? 12 : 8;
     const SolveGrid g = solve_grid(plan.m, rec_bytes, ctx->sm_count, ctx->tune_edge_ctas);
     a.seg = seg_records(plan.m, g.blocks * (uint32_t)(g.threads / 32), rec_bytes);
-    PHEM_CUDA_TRY(cudaMemsetAsync(ctx->ctl, 0, sizeof(Ctl), st));
+    PHEM_TRY(solve_ctl(ctx, &a.ctl, &a.publish));
     void *params[] = {&a};
     KernelScope ks(ctx, kKSolve);
     if (g.blocks == 1)  // one CTA waits for no other
@@ -701,13 +754,38 @@ uint64_t list_capacity(uint64_t m, int sm_count)
     return m + ((uint64_t)sm_count * kSolveWarps + 1) * (kEpStageBytes / 8);
 }
 
+phem_status solve_ctl(phem_context *ctx, Ctl **ctl, Ctl **publish)
+{
+    ctx->publishes = !ctx->profiling;  // a profiled solve's time stamps stay in the block
+    *ctl = ctx->publishes ? ctx->solve_ctl : ctx->ctl;
+    *publish = ctx->publishes ? ctx->h_ctl : nullptr;
+    if (!ctx->publishes || !ctx->solve_ctl_zero)
+        PHEM_CUDA_TRY(cudaMemsetAsync(*ctl, 0, sizeof(Ctl), ctx->stream));
+    if (ctx->publishes) {
+        ctx->solve_ctl_zero = false;
+        ctx->h_ctl->err = kCtlPending;
+    }
+    return PHEM_OK;
+}
+
 phem_status msf_finish(phem_context *ctx, uint32_t *rounds_out, const char *what)
 {
-    PHEM_CUDA_TRY(cudaMemcpyAsync(ctx->h_ctl, ctx->ctl, ctx->profiling ? sizeof(Ctl) : offsetof(Ctl, bar),
-                                  cudaMemcpyDeviceToHost, ctx->stream));
+    const bool published = ctx->publishes;
+    ctx->publishes = false;
+    if (!published)
+        PHEM_CUDA_TRY(cudaMemcpyAsync(ctx->h_ctl, ctx->ctl, ctx->profiling ? sizeof(Ctl) : offsetof(Ctl, bar),
+                                      cudaMemcpyDeviceToHost, ctx->stream));
     PHEM_TRY(stream_wait(ctx));
     const Ctl &h = *ctx->h_ctl;
-    if (ctx->profiling)
+    if (published) {
+        ctx->solve_ctl_zero = h.err != kCtlPending;
+        if (!ctx->solve_ctl_zero) {  // gave up at a barrier
+            PHEM_CUDA_TRY(cudaMemcpyAsync(ctx->h_ctl, ctx->solve_ctl, offsetof(Ctl, bar), cudaMemcpyDeviceToHost,
+                                          ctx->stream));
+            PHEM_TRY(stream_wait(ctx));
+        }
+    }
+    if (!published && ctx->profiling)
         for (uint32_t i = 1; i < h.stamps && i < kMaxPhases; i++)
             log_phase(ctx, (int)h.phase_of[i], (float)(h.stamp[i] - h.stamp[i - 1]) * 1e-6f);
     if (rounds_out)
@@ -756,6 +834,7 @@ phem_status msf_plan(phem_context *ctx, const void *d_e0, uint64_t m, uint32_t n
     plan->m = m;
     plan->n = n;
     plan->forest = nullptr;
+    plan->label = nullptr;
     plan->out = nullptr;
     plan->gather = 0;
     if (extra_off)

@@ -360,3 +360,37 @@ def test_device_edges_in_rounds(ctx, kind, odd):
         with pytest.raises(P.PhemError) as ei:
             ctx.cc_solve(bad, n, labels=lab, forest=slots)
         assert ei.value.status == _lib.PHEM_ERR_INVALID
+
+
+@pytest.mark.parametrize("n", [20000, 40003])
+def test_solves_after_failed_and_profiled_ones(ctx, n):
+    """A solve hands over a zeroed control block: canonical CC, weighted MSF
+    and default CC repeated in turn, after solves that gave up on an endpoint
+    out of range and with profiled ones (another control block) in between."""
+    p = gen.er(n, 3 * n + 1, 9)
+    want, _ = oracle.cc_solve(p, n)
+    cset = forest_set(ctx.cc_solve(p, n, canonical=True).forest)
+    w = np.random.default_rng(1).integers(0, 1000, len(p), dtype=np.uint32)
+    e = np.stack([(p >> np.uint64(32)).astype(np.uint32), p.astype(np.uint32), w], axis=1)
+    flags, cnt, tot = oracle.msf_kruskal(e, n)
+    bad_p, bad_e = p.copy(), e.copy()
+    bad_p[-1] = np.uint64((3 << 32) | n)
+    bad_e[-1, 1] = n
+    for step in range(4):
+        if step % 2:
+            for call in (lambda: ctx.msf_solve(bad_e, n), lambda: ctx.cc_solve(bad_p, n, canonical=True),
+                         lambda: ctx.cc_solve(bad_p, n)):
+                with pytest.raises(P.PhemError):
+                    call()
+        ctx.set_profiling(step == 2)
+        r = ctx.msf_solve(e, n)
+        assert (r.count, r.total) == (cnt, tot)
+        np.testing.assert_array_equal(r.edges, e[flags])
+        c = ctx.cc_solve(p, n, canonical=True)
+        np.testing.assert_array_equal(c.labels, want)
+        np.testing.assert_array_equal(forest_set(c.forest), cset)
+        assert c.components == len(np.unique(want)) == n - c.forest_edges
+        d = ctx.cc_solve(p, n)
+        np.testing.assert_array_equal(d.labels, want)
+        assert d.components == c.components
+        ctx.set_profiling(False)
