@@ -666,13 +666,16 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
     if (s <= 0 || s >= m)
         s = m;
     // edges on the device are solved in one launch, whose lists hold the
-    // prefix (a much longer one than usual stays with the launches below)
-    const bool one_launch = !canonical && !overlap && s <= 4 * (int64_t)n + (1 << 20);
-    const size_t extra = o_par + (one_launch ? cc_grid_bytes(m, s, n, ctx->sm_count) : align256(lb));
+    // prefix (a much longer one than usual stays with the launches below,
+    // and one that must keep to a scratch limit that the lists would exceed)
+    const size_t grid_extra = o_par + cc_grid_bytes(m, s, n, ctx->sm_count);
+    const bool one_launch = !canonical && !overlap && s <= 4 * (int64_t)n + (1 << 20) &&
+                            (!ctx->scratch_limit || grid_extra <= ctx->scratch_limit);
+    const size_t extra = one_launch ? grid_extra : o_par + align256(lb);
     size_t base = 0;
     MsfPlan plan;
     if (canonical) {
-        PHEM_TRY(msf_plan(ctx, nullptr, (uint64_t)m, (uint32_t)n, extra, &plan, &base));
+        PHEM_TRY(msf_plan(ctx, kKindPacked, (uint64_t)m, (uint32_t)n, extra, 0, &plan, &base));
     } else {
         PHEM_TRY(ws_reserve(ctx, extra));
     }
@@ -1038,7 +1041,7 @@ static phem_status msf_common(phem_context *ctx, const phem_edge *edges, uint64_
     const size_t o_edges = 0, o_out = aligned_dev ? 0 : align256(eb);  // edges read in place: no staging area
     size_t base = 0;
     MsfPlan plan;
-    PHEM_TRY(msf_plan(ctx, nullptr, m, n, o_out + align256(ob), &plan, &base));
+    PHEM_TRY(msf_plan(ctx, kKindMsf, m, n, o_out + align256(ob), o_out, &plan, &base));
     Staged se, so;
     if (aligned_dev) {
         se.dev = const_cast<phem_edge *>(edges);
@@ -1162,8 +1165,7 @@ static phem_status msf_stream_impl(phem_context *ctx, const phem_edge *h_edges, 
         // size the solve workspace once for the largest solve (a later growth
         // would free memory, which waits for the copies in flight)
         MsfPlan plan;
-        PHEM_TRY(msf_plan(ctx, nullptr, R + top, n, align256((size_t)n * sizeof(phem_edge)), &plan,
-                          nullptr));
+        PHEM_TRY(msf_plan(ctx, kKindMsf, R + top, n, align256((size_t)n * sizeof(phem_edge)), 0, &plan, nullptr));
     }
     char *b = static_cast<char *>(ctx->input);
     phem_edge *slot[2] = {reinterpret_cast<phem_edge *>(b), reinterpret_cast<phem_edge *>(b + slot_bytes)};

@@ -63,6 +63,7 @@ struct phem_context {
     uint32_t tiny_ready = 0;           // bit k: launch attributes of small-solve kernel k are set
     uint64_t epoch = 1;                // look-back epoch counter
     uint32_t timeout_ms = 0;
+    size_t scratch_limit = 0;          // workspace bytes a CC solve keeps to by its choice of path (0: none)
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
     uint32_t kernels_ready = 0;        // bit k: launch attributes of edge kind k are set
     int tune_edge_ctas = 4;              // MSF solve: groups of 8 independent warps per SM, 1 to 4
@@ -272,8 +273,11 @@ struct MsfPlan {
 // The canonical forest's light edges (the first ones by index; 0: no split).
 uint64_t canonical_light(phem_context *ctx, uint64_t m, uint64_t n);
 size_t msf_workspace_bytes(uint64_t m, uint32_t n, int sm_count);
-phem_status msf_plan(phem_context *ctx, const void *d_e0, uint64_t m, uint32_t n, size_t extra_bytes, MsfPlan *plan,
-                     size_t *extra_off);
+// Reserves and carves the workspace; *extra_off: the caller's extra_bytes in
+// it.  kKindMsf: the n records at extra offset out_off are written only by
+// the gather, and hold round state before it.
+phem_status msf_plan(phem_context *ctx, int kind, uint64_t m, uint32_t n, size_t extra_bytes, size_t out_off,
+                     MsfPlan *plan, size_t *extra_off);
 // Queues the whole solve (one launch); msf_finish waits and checks.
 phem_status msf_run(phem_context *ctx, int kind, MsfPlan &plan);
 // The control block of the solve about to be queued, zero when its kernels

@@ -794,13 +794,16 @@ phem_status msf_finish(phem_context *ctx, uint32_t *rounds_out, const char *what
 }
 
 // Workspace of one solve (msf_plan carves in the same order): parent (4n),
-// best (2 x 8n), the MSF bitmap (m / 8), the giant bits (n / 8) and the
-// survivor segments (16 bytes per record).
-static size_t msf_carve(uint64_t m, uint32_t n, int sm_count, char *base, MsfPlan *p)
+// best (8n), the MSF bitmap (m / 8), the giant bits (n / 8) and the survivor
+// segments (20 bytes per record), then the caller's extra area.  The second
+// best array of a weighted solve lies in the extra area's start, where the
+// staged MSF records go (12n): they are written behind the rounds.  The packed
+// kind's extra area holds arrays that the rounds write, so it gets its own.
+static size_t msf_carve(uint64_t m, uint32_t n, int sm_count, int bests, char *base, MsfPlan *p)
 {
     Carve c;
     const uint64_t stride = ((uint64_t)n + 31) & ~31ull;
-    const size_t o_par = c.take<uint32_t>(n), o_best = c.take<unsigned long long>(2 * stride),
+    const size_t o_par = c.take<uint32_t>(n), o_best = c.take<unsigned long long>(bests * stride),
                  o_samp = c.take<uint32_t>(2 * kMaxSample), o_bm = c.take<uint32_t>((m + 31) / 32 + 4),
                  o_cnt = c.take<uint32_t>(gather_chunks(m) + 4), o_tot = c.take<uint32_t>(kMaxGrid),
                  o_gi = c.take<uint32_t>(stride / 32 + 4), o_list = c.take<uint4>(list_capacity(m, sm_count)),
@@ -820,17 +823,25 @@ static size_t msf_carve(uint64_t m, uint32_t n, int sm_count, char *base, MsfPla
     return c.off;
 }
 
-size_t msf_workspace_bytes(uint64_t m, uint32_t n, int sm_count) { return msf_carve(m, n, sm_count, nullptr, nullptr); }
-
-phem_status msf_plan(phem_context *ctx, const void *d_e0, uint64_t m, uint32_t n, size_t extra_bytes, MsfPlan *plan,
-                     size_t *extra_off)
+size_t msf_workspace_bytes(uint64_t m, uint32_t n, int sm_count)
 {
+    return msf_carve(m, n, sm_count, 1, nullptr, nullptr);
+}
+
+phem_status msf_plan(phem_context *ctx, int kind, uint64_t m, uint32_t n, size_t extra_bytes, size_t out_off,
+                     MsfPlan *plan, size_t *extra_off)
+{
+    const int bests = kind == kKindMsf ? 1 : 2;
+    const size_t second = bests == 1 ? out_off + 8 * (((size_t)n + 31) & ~size_t(31)) : 0;
     Carve c;
-    c.off = msf_workspace_bytes(m, n, ctx->sm_count);
-    const size_t extra_at = c.take<uint8_t>(extra_bytes);
+    c.off = msf_carve(m, n, ctx->sm_count, bests, nullptr, nullptr);
+    const size_t extra_at = c.take<uint8_t>(std::max(extra_bytes, second));
     PHEM_TRY(ws_reserve(ctx, c.off));
-    msf_carve(m, n, ctx->sm_count, static_cast<char *>(ctx->ws), plan);
-    plan->e0 = d_e0;
+    msf_carve(m, n, ctx->sm_count, bests, static_cast<char *>(ctx->ws), plan);
+    if (bests == 1)
+        plan->best_stride = (extra_at + out_off - (reinterpret_cast<char *>(plan->best) - static_cast<char *>(ctx->ws))) /
+                            sizeof(unsigned long long);
+    plan->e0 = nullptr;
     plan->m = m;
     plan->n = n;
     plan->forest = nullptr;

@@ -402,8 +402,10 @@ phem_status phem_server_create(int device, const phem_server_config *cfg, phem_s
     for (uint32_t k = 0; st == PHEM_OK && k < cfg->large_workers; k++) {
         phem_context *c = nullptr;
         st = phem_context_create(device, &c);
-        if (st == PHEM_OK)
+        if (st == PHEM_OK) {
+            c->scratch_limit = s->large_share;
             s->large_ctx.push_back(c);
+        }
     }
     // re-capture every slot's launch with its CC pairs buffer wired in
     for (auto &sl : s->slots) {

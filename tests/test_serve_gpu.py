@@ -7,7 +7,7 @@ import threading
 import numpy as np
 import pytest
 
-from phem_graph_b200 import _lib
+from phem_graph_b200 import _lib, gen
 from phem_graph_b200._lib import PhemError
 from phem_graph_b200.serve import (PHEM_BATCH_CC, PHEM_BATCH_MSF, Server, ServedGraph, poisson_arrivals,
                                    request_pool)
@@ -81,6 +81,16 @@ def test_budget_refuses_what_never_fits():
         small = ServedGraph(PHEM_BATCH_CC, 4, pairs=np.array([1, (2 << 32) | 3], np.uint64))
         s = srv.solve(small)
         np.testing.assert_array_equal(s.labels, [0, 0, 2, 2])
+
+
+@pytest.mark.parametrize("n", [600000, 1500000])
+def test_large_cc_keeps_to_its_share(ctx, n):
+    """Requests that the share admits but whose prefix lists it would not
+    hold are solved without the lists, with the same labels."""
+    with Server(memory_budget=68 << 20, slots=1, max_batch_graphs=8, large_edges=1 << 10, large_workers=1) as srv:
+        pairs = gen.er(n, 700000, 5)
+        s = srv.solve(ServedGraph(PHEM_BATCH_CC, n, pairs=pairs))
+        np.testing.assert_array_equal(s.labels, ctx.cc_solve(pairs, n).labels)
 
 
 def test_bad_requests_fail_alone():
