@@ -15,8 +15,10 @@
 //   4. csr_pass_kernel<kPairs or kRecords> resolves the rows again and writes
 //      the kept entries in order: group offset + segment offset + the lanes
 //      before.  The record form fuses the MSF CSR input's packing: the
-//      kept entry at position p becomes {row, col, w[p]}; a warp's records are
-//      put together in shared memory and leave as 16-byte stores.
+//      kept entry at position p becomes {row, col, w[p]}; a warp's pairs or
+//      records are put together in shared memory and leave as 16-byte stores
+//      (pairs by 8-byte stores from the lanes, four times the L2 sectors:
+//      R-MAT 20 212 us per call against 177).
 // Every entry keeps its place in the reference's row walk, so the output order
 // (and therefore the edge numbering) is exactly the reference's.  The next
 // segment's columns and row range are loaded while the current one is worked
@@ -52,8 +54,10 @@ enum CsrMode : int { kCount = 0, kPairs, kRecords };
 // A row of many segments is written by its whole warp.  Malformed offsets
 // leave segments unwritten; the conversion clamps what it reads.
 __global__ void __launch_bounds__(kBlock) csr_seg_rows_kernel(const int64_t *offsets, int32_t n, uint32_t nseg,
-                                                              uint32_t *seg_rows)
+                                                              uint32_t *seg_rows, unsigned long long *ticket)
 {
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        *ticket = 0;  // of the scan, two launches on
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const uint32_t lane = lane_id();
     for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x; i0 < n; i0 += stride) {
@@ -184,7 +188,7 @@ __global__ void __launch_bounds__(kCsrThreads, csr_blocks_per_sm(MODE))
                     const uint32_t *w, phem_edge *rec_out, uint64_t cap)
 {
     __shared__ __align__(16) uint32_t s_mark[kCsrWarps][kCsrSeg];
-    __shared__ __align__(16) uint32_t s_out[kCsrWarps][MODE == kRecords ? kCsrSeg * 3 + 4 : 4];
+    __shared__ __align__(16) uint32_t s_out[kCsrWarps][MODE == kRecords ? kCsrSeg * 3 + 4 : MODE == kPairs ? kCsrSeg * 2 + 4 : 4];
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     const bool wide = ((uintptr_t)cols & 15) == 0;
     const uint32_t nseg = (uint32_t)((nnz + kCsrSeg - 1) / kCsrSeg);
@@ -226,10 +230,27 @@ __global__ void __launch_bounds__(kCsrThreads, csr_blocks_per_sm(MODE))
         uint32_t total = __shfl_sync(0xffffffffu, at, 31);
         at -= own;
         if (MODE == kPairs) {
+            // as the records below, in 16-byte stores of two pairs
+            const uint32_t shift = (uint32_t)((reinterpret_cast<uintptr_t>(out) >> 3) + base) & 1u;
+            unsigned long long *so = reinterpret_cast<unsigned long long *>(s_out[warp]);
 #pragma unroll
             for (int k = 0; k < kCsrItems; k++)
                 if (keep >> k & 1)
-                    out[base + at++] = ((unsigned long long)row[k] << 32) | col[k];
+                    so[shift + at++] = ((unsigned long long)row[k] << 32) | col[k];
+            __syncwarp();
+            const uint32_t end = shift + total;
+            unsigned long long *g = out + base - shift;
+            for (uint32_t c = lane * 2; c < end; c += 64) {
+                const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(so + c);
+                if (c >= shift && c + 2 <= end) {
+                    __stcs(reinterpret_cast<ulonglong2 *>(g + c), v);
+                } else {
+                    if (c >= shift)
+                        g[c] = v.x;
+                    if (c + 1 >= shift && c + 1 < end)
+                        g[c + 1] = v.y;
+                }
+            }
             continue;
         }
         if (base + total > cap)  // a wrong entry count: only the first cap records are written
@@ -339,8 +360,6 @@ __global__ void __launch_bounds__(kScanBlock) csr_scan_kernel(const uint32_t *co
     if (!s_last)
         return;
     __threadfence();
-    if (threadIdx.x == 0)
-        *ticket = 0;
     uint64_t carry = 0;
     for (uint32_t g0 = 0; g0 < gridDim.x; g0 += kScanBlock) {
         const uint32_t g = g0 + threadIdx.x;
@@ -393,10 +412,10 @@ phem_status csr_launch_to_coo(phem_context *ctx, const int64_t *offsets, const u
         KernelScope k(ctx, kKCsrCoo);
         const int rblocks = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)n + kBlock - 1) / kBlock,
                                                                          (int64_t)ctx->sm_count * 8));
-        csr_seg_rows_kernel<<<rblocks, kBlock, 0, ctx->stream>>>(offsets, n, (uint32_t)segs, seg_rows);
+        csr_seg_rows_kernel<<<rblocks, kBlock, 0, ctx->stream>>>(offsets, n, (uint32_t)segs, seg_rows,
+                                                                &ctx->ctl->misc[3]);
     }
     pass(csr_pass_kernel<kCount>, kCount);
-    PHEM_CUDA_TRY(cudaMemsetAsync(&ctx->ctl->misc[3], 0, sizeof(unsigned long long), ctx->stream));  // scan ticket
     {
         KernelScope k(ctx, kKCsrCoo);
         csr_scan_kernel<<<(unsigned)groups, kScanBlock, 0, ctx->stream>>>(counts, (uint32_t)segs, prefix, group_tot,

@@ -416,3 +416,24 @@ def test_csr_segments(ctx, kind, skew):
     d_w = torch.from_numpy(w.view(np.int32)).cuda()
     torch.cuda.synchronize()
     assert_msf(ctx.msf_solve_csr(d_off, d_cols, n, d_w, len(want)), E, ids, cnt, tot)
+
+
+@pytest.mark.parametrize("at", [0, 1])
+@pytest.mark.parametrize("length", [1, 2, 255, 257, 5000])
+def test_csr_pairs_at_any_offset(ctx, at, length):
+    """Pairs leave as 16-byte stores from either 8-byte offset, and nothing is
+    written around them."""
+    import torch
+    n = length + 1
+    off, cols = _csr_from_entries(np.zeros(length, np.int64), np.arange(1, n), n)
+    want = oracle.csr_to_coo(off, cols, n)
+    d_off, d_cols = torch.from_numpy(off).cuda(), torch.from_numpy(cols.view(np.int32)).cuda()
+    d_out = torch.full((length + 4,), -7, dtype=torch.int64, device="cuda")
+    k = _lib.C.c_int64()
+    torch.cuda.synchronize()
+    _lib.check(_lib.lib().phem_csr_to_coo(ctx._h, d_off.data_ptr(), d_cols.data_ptr(), n,
+                                          d_out[1 + at:].data_ptr(), _lib.C.byref(k)), "phem_csr_to_coo")
+    got = d_out.cpu().numpy()
+    assert k.value == len(want) == length
+    np.testing.assert_array_equal(got[1 + at:1 + at + length].view(np.uint64), want)
+    assert (got[:1 + at] == -7).all() and (got[1 + at + length:] == -7).all()
