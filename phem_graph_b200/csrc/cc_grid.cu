@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) cc_grid_kernel(const __grid_
     clock.stamp(kKCcUnite);
     // a hooked vertex's forest edge is the one to the parent it got; then
     // every vertex to its root
-    full_compress(a.parent, a.n, nullptr, nullptr, 0, false, &ctl->err, a.forest);
+    full_compress<true>(a.parent, a.n, nullptr, nullptr, 0, false, &ctl->err, a.forest);
     if (!grid_sync(ctl, s, seq))
         return;
     clock.stamp(kKCcLabel);

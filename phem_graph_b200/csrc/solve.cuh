@@ -487,7 +487,10 @@ __device__ __forceinline__ void compress_pass(uint32_t *parent, uint32_t n, uint
 // relabels endpoints in one hop) and the roots' next best words reset (when
 // best_next is set); with use_giant also one bit per vertex: in the component
 // of root `giant`; with forest also every vertex's forest slot, the edge to
-// the parent it had.
+// the parent it had.  CHAINS: the pointers may form chains as long as the
+// graph (a path whose every vertex hooked under the one before it), which are
+// shortened from all sides as in compress_pass.
+template <bool CHAINS = false>
 __device__ __forceinline__ void full_compress(uint32_t *parent, uint32_t n, unsigned long long *best_next,
                                               uint32_t *bits_of, uint32_t giant, bool use_giant, uint32_t *err,
                                               unsigned long long *forest = nullptr)
@@ -512,11 +515,14 @@ __device__ __forceinline__ void full_compress(uint32_t *parent, uint32_t n, unsi
             uint32_t p[kVItems];
 #pragma unroll
             for (int k = 0; k < kVItems; k++)
-                p[k] = walking[k] ? ld_par(parent + y[k]) : y[k];
+                p[k] = !walking[k] ? y[k]
+                                   : (CHAINS && steps >= 8 ? __ldcg(parent + y[k]) : ld_par(parent + y[k]));
             bool any = false;
 #pragma unroll
             for (int k = 0; k < kVItems; k++) {
                 walking[k] = walking[k] && p[k] != y[k];
+                if (CHAINS && steps >= 8 && walking[k])
+                    parent[x[k]] = p[k];
                 y[k] = p[k];
                 any |= walking[k];
             }
