@@ -475,8 +475,11 @@ __global__ void __launch_bounds__(kBlock) cc_regroup_kernel(const __grid_constan
         a.ctl->misc[5] = root;
 }
 
-// Labels (every vertex to its root) and the number of components.
-__global__ void __launch_bounds__(kBlock) cc_label_count_kernel(const __grid_constant__ CcArgs a)
+// Labels (every vertex to its root) and the number of components.  Bound by
+// the walks' L2 latency, so by the warps in flight: two blocks per SM (102
+// registers) / four (64), us per call: n = 2^21 282 / 275, R-MAT 22 361 / 355;
+// six and eight the same as four.
+__global__ void __launch_bounds__(kBlock, 4) cc_label_count_kernel(const __grid_constant__ CcArgs a)
 {
     __shared__ unsigned long long s_roots;
     if (threadIdx.x == 0)
