@@ -251,8 +251,8 @@ phem_status phem_cc_merge(phem_context *ctx, const uint64_t *d_forest_a, const u
 #define PHEM_CC_NOALLOC_MAX_VERTICES (1 << 20)
 
 /* CC + spanning forest that allocates nothing.  No counterpart in the
- * reference: it is phem_cc_solve's default path (same labels, a forest of the
- * same kind) for callers that cannot allocate device memory at solve time --
+ * reference: phem_cc_solve's default mode (same labels, a forest of the same
+ * kind) for callers that cannot allocate device memory at solve time --
  * a serving process whose memory is committed under a budget, or a loop that
  * cannot afford cudaMalloc/cudaFree stalling the device -- and so takes no
  * context either.  The parent array lives in fixed static device scratch.

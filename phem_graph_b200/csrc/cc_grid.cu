@@ -27,7 +27,7 @@
 // The labels array is the parent array: the last compress leaves the labels.
 //
 // us per call, before (cc.cu's launches) -> now: uniform n = 2,000,003, m = 2^23
-// 420 -> 290, R-MAT 22 (67 M edges) 440 -> 360.  Bound: the rest's gathers and
+// 450 -> 275, R-MAT 22 (67 M edges) 444 -> 355.  Bound: the rest's gathers and
 // bits (64% L1 hits, 47% of the L2 sector rate, 56% of the issue slots on R-MAT
 // 21) and, for uniform graphs, the scattered accesses of the rounds.
 #include <algorithm>

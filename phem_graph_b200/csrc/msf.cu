@@ -44,10 +44,10 @@
 // finds nothing to do) and the list's trip through memory cost more than the
 // work; a grid barrier costs 1.2 us, and lists private to a warp need no
 // reservation.  Against the same phases as separate launches (one per phase
-// and round, shared lists): n = 131,101, m = 2^20 uniform 592 -> 287 us; n =
-// 262,147 geometric 645 -> 315 us; R-MAT 22 (67 M edges) 1314 -> 1053 us;
-// n = 2,003, m = 8,009 312 -> 159 us; the canonical forest of n = 2^20,
-// m = 2^23 943 -> 543 us.  Walking parent[] in the edge pass instead of the
+// and round, shared lists), us per call, then with what the comments below
+// measure: n = 131,101, m = 2^20 uniform 592 -> 287 -> 211; n = 262,147
+// geometric 645 -> 315 -> 273; R-MAT 22 (67 M edges) 1314 -> 1053 -> 980; the
+// canonical forest of n = 2^20, m = 2^23 943 -> 543 -> 514.  Walking parent[] in the edge pass instead of the
 // separate compress phase cost 3344 us on R-MAT 22: the path-halving stores
 // of every record of a hub hit one word.
 #include <algorithm>

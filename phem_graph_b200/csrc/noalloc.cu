@@ -1,8 +1,9 @@
 // noalloc.cu -- connected components + spanning forest without allocating.
 //
-// phem_cc_solve_noalloc runs phem_cc_solve's union-find (the same union
-// steps, uf.cuh, and the same prefix / compress / rest schedule), so its
-// labels and forest mean the same (the reference's
+// phem_cc_solve_noalloc runs the union-find of cc.cu (the same union steps,
+// uf.cuh, and the same prefix / compress / rest schedule), which needs no
+// scratch beside the parents; labels and forest mean what phem_cc_solve's do
+// (the reference's
 // init_parent_label_T1edges + union_find_gpu_COO + cc,
 // CC/ExternalSpanningTree.cu:77-116, CC/GPUSpanningTree.cu:122-128), with its
 // parent array in a fixed-size file-scope device array instead of a context
@@ -61,7 +62,7 @@ __global__ void __launch_bounds__(kBlock) na_init_kernel(int32_t n, int32_t *par
 }
 
 // Two packed edges per 128-bit streaming load (edges 16-byte aligned), the
-// odd last edge alone; the union is phem_cc_solve's (uf.cuh).
+// odd last edge alone; the union is cc.cu's (uf.cuh).
 __global__ void __launch_bounds__(kBlock) na_unite_kernel(const unsigned long long *edges, int64_t m, int32_t n,
                                                           int32_t *parent, unsigned long long *forest,
                                                           uint32_t *status)
@@ -167,7 +168,7 @@ extern "C" phem_status phem_cc_solve_noalloc(const uint64_t *d_edges, int64_t m,
 
     na_init_kernel<<<na_grid(sm_count, n), kBlock, 0, st>>>(n, s.parent, forest, s.status);
     PHEM_CUDA_TRY(cudaGetLastError());
-    // phem_cc_solve's schedule: a prefix of about one edge per vertex builds
+    // the schedule of cc.cu: a prefix of about one edge per vertex builds
     // the big components, a compress points every vertex at its root, then
     // the rest of the edges (an even prefix keeps the rest 16-byte aligned)
     const unsigned long long *e = reinterpret_cast<const unsigned long long *>(d_edges);
