@@ -541,28 +541,33 @@ GridHdr batch_grid_items(const BatchItem *items, uint32_t G, GridItem *out)
 // Which kernel takes a batch: the one whose time, from these measured rates,
 // is shorter.  The CTA-per-graph kernel ends with its largest graph (4.5 ns per
 // edge or vertex with the state in shared memory, 10 ns without) or when its
-// two CTAs per SM have worked everything off (12 ns each, 25 us per graph);
+// two CTAs per SM have worked everything off (12 ns per edge or vertex of a
+// graph with its state in shared memory, 18 ns otherwise, 25 us per graph);
 // the grid pays its barriers once and 55 ps per edge or vertex.  us, CTA per
 // graph / grid: 256 graphs of up to 65,536 vertices (16.7 M edges and vertices)
 // 5608 / 1117, of up to 8192 566 / 353, of up to 4096 215 / 282; 4 of up to
-// 20,000 468 / 182; 4096 of up to 128 451 / 196, of up to 4096 1143 / 1198.
+// 20,000 468 / 182; 2048 of up to 8192 1033 / 1144; 4096 of up to 128 451 /
+// 196, of up to 4096 1143 / 1198, of up to 16,384 3829 / 3270, of up to 65,536
+// (215 M) 15,045 / 9618.
 bool batch_takes_grid(const BatchLayout &L, int sm_count)
 {
     constexpr uint32_t kCtaSmemVertices = 5700;  // with the default configuration
-    double all = 0, largest = 0;
+    double all = 0, cta = 0, largest = 0;
     uint64_t verts = 0;
     for (const BatchItem &x : L.items) {
         if (x.kind == kBatchPairs)
             return false;
         const double work = (double)x.m + x.n;
+        const bool smem = x.n <= kCtaSmemVertices;
         all += work;
-        largest = std::max(largest, work * (x.n <= kCtaSmemVertices ? 4.5 : 10.0));
+        cta += work * (smem ? 12.0 : 18.0) + 25e3;
+        largest = std::max(largest, work * (smem ? 4.5 : 10.0));
         verts += ((uint64_t)x.n + 31) & ~31ull;
     }
     const uint64_t tiles = L.wl_records / kTileRecs + 2ull * L.items.size();
     if (tiles * kTileRecs >= (1ull << 32) - (1u << 24) || verts >= (1ull << 31))
         return false;  // union ids and vertices are 32-bit
-    const double cta_ns = 25e3 + std::max(largest, (12.0 * all + 25e3 * (double)L.items.size()) / (2.0 * sm_count));
+    const double cta_ns = 25e3 + std::max(largest, cta / (2.0 * sm_count));
     const double grid_ns = 190e3 + 0.055 * all;
     return grid_ns < cta_ns;
 }
