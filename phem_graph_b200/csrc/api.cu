@@ -666,11 +666,11 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
     if (s <= 0 || s >= m)
         s = m;
     // edges on the device are solved in one launch, whose lists hold the
-    // prefix (a much longer one than usual stays with the launches below,
-    // and one that must keep to a scratch limit that the lists would exceed)
-    const size_t grid_extra = o_par + cc_grid_bytes(m, s, n, ctx->sm_count);
-    const bool one_launch = !canonical && !overlap && s <= 4 * (int64_t)n + (1 << 20) &&
-                            (!ctx->scratch_limit || grid_extra <= ctx->scratch_limit);
+    // prefix (a much longer one than usual stays with the launches below).  A
+    // server's workers keep to the launches: they need no lists, which the
+    // admission of requests does not count, and no SMs all at once (run_impl)
+    const bool one_launch = !canonical && !overlap && !ctx->shares_device && s <= 4 * (int64_t)n + (1 << 20);
+    const size_t grid_extra = o_par + (one_launch ? cc_grid_bytes(m, s, n, ctx->sm_count) : 0);
     const size_t extra = one_launch ? grid_extra : o_par + align256(lb);
     size_t base = 0;
     MsfPlan plan;

@@ -21,7 +21,7 @@
 //   * phem_cc_solve unites a prefix of about one edge per vertex, points
 //     every vertex at its root, then unites the rest (cc.sample_per_vertex);
 //     these kernels do it for host edges that are copied in chunks, for the
-//     stage and streaming entry points and where a scratch limit or a long
+//     stage and streaming entry points, for a server's workers and where a long
 //     prefix excludes the lists of cc_grid.cu, which solves everything else;
 //   * every loop is bounded; a bound that trips sets a status bit instead of
 //     hanging the GPU.

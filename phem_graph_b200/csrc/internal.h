@@ -63,7 +63,7 @@ struct phem_context {
     uint32_t tiny_ready = 0;           // bit k: launch attributes of small-solve kernel k are set
     uint64_t epoch = 1;                // look-back epoch counter
     uint32_t timeout_ms = 0;
-    size_t scratch_limit = 0;          // workspace bytes a CC solve keeps to by its choice of path (0: none)
+    bool shares_device = false;        // other contexts' work runs beside this one's (a server's workers)
     cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
     uint32_t kernels_ready = 0;        // bit k: launch attributes of edge kind k are set
     int tune_edge_ctas = 4;              // MSF solve: groups of 8 independent warps per SM, 1 to 4

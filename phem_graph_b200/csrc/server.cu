@@ -403,7 +403,7 @@ phem_status phem_server_create(int device, const phem_server_config *cfg, phem_s
         phem_context *c = nullptr;
         st = phem_context_create(device, &c);
         if (st == PHEM_OK) {
-            c->scratch_limit = s->large_share;
+            c->shares_device = true;
             s->large_ctx.push_back(c);
         }
     }
