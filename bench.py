@@ -390,15 +390,14 @@ def bench_batched(ctx, torch, num_graphs: int = 4096) -> dict:
             "vertices": b.total_vertices, "unit": UNIT, "value": b.total_edges / (ms / 1e3) / 1e9,
             "ms_per_batch": ms, "graphs_per_s": b.num_graphs / (ms / 1e3), "launches_per_batch": 1,
             "config": {k: tuned[k] for k in ("block_size", "items", "compact_ratio", "grid", "smem_vertices")},
-            "replay": "captured CUDA graph (queue reset + persistent kernel)",
+            "replay": "captured CUDA graph (both batch kernels; the one the batch is not for returns at once)",
             "one_launch_per_graph": {"value": b.total_edges / plain_batch_s / 1e9, "s_per_batch": plain_batch_s,
                                      "sample": "256 graphs through phem_msf_solve, scaled by edge share"},
             "speedup_vs_one_launch_per_graph": plain_batch_s / (ms / 1e3),
             "one_launch_per_graph_device": {"value": b.total_edges / dev_batch_s / 1e9, "s_per_batch": dev_batch_s,
                                             "sample": "the same 256 graphs resident on the device, one "
                                                       "phem_msf_solve_device per graph, scaled by edge share; "
-                                                      "that path waits on the host between round batches, so "
-                                                      "it has no captured form"},
+                                                      "each call waits for its own result"},
             "speedup_vs_one_launch_per_graph_device": dev_batch_s / (ms / 1e3),
             "e2e": {"value": b.total_edges / e2e / 1e9, "unit": UNIT, "ms_per_step": e2e * 1e3,
                     "h2d_bytes_per_step": 12 * b.total_edges + 24 * b.num_graphs,
