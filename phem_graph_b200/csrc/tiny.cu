@@ -5,9 +5,9 @@
 // are the time, not the work.  Here one CTA of 1024 threads holds the graph:
 // every thread keeps K edge records in registers for the whole solve (record
 // k * 1024 + thread, so its id is implied and a record never moves), and the
-// per-vertex state lives in shared memory.  Host inputs are read in place
-// from pinned staging memory and results are written to it, so a host call
-// makes no copy of its own; the control block's results go straight to its
+// per-vertex state lives in shared memory.  Host inputs are read in place from
+// pinned memory (the caller's, or staging for a pageable array) and results are
+// written to it, so a host call queues no copy of its own; the control block's results go straight to its
 // pinned mirror.
 //
 // Bound: shared-memory gathers.  A live record costs four per round (its two
@@ -479,13 +479,18 @@ phem_status tiny_input(phem_context *ctx, const void *p, size_t bytes, void *ws,
     }
     if (attr.type == cudaMemoryTypeDevice && attr.device == ctx->device && ((uintptr_t)p & 3) == 0)
         return PHEM_OK;
-    if (attr.type == cudaMemoryTypeUnregistered || attr.type == cudaMemoryTypeHost) {
+    if (attr.type == cudaMemoryTypeHost && attr.devicePointer && ((uintptr_t)p & 7) == 0) {
+        *in = attr.devicePointer;
+        return PHEM_OK;
+    }
+    if (attr.type == cudaMemoryTypeUnregistered && cudaStreamQuery(ctx->stream) == cudaSuccess) {
         char *buf = nullptr;
         PHEM_TRY(tiny_host(ctx, &buf));
         std::memcpy(buf, p, bytes);
         *in = buf;
         return PHEM_OK;
     }
+    cudaGetLastError();  // "not ready" is no error
     *in = ws;
     PHEM_CUDA_TRY(cudaMemcpyAsync(ws, p, bytes, cudaMemcpyDefault, ctx->stream));
     return PHEM_OK;

@@ -15,14 +15,17 @@ constexpr uint32_t kTinyCcMaxEdges = 32768, kTinyCcMaxVertices = 32768;
 static_assert(kTinyCcMaxEdges * 8 >= kTinyMaxEdges * 12, "the staging buffer's input part holds either kind");
 constexpr size_t kTinyDynSmem = 16384 * 12 + 16;
 
-// The context's pinned staging buffer: a small solve's host input at 0, its
+// The context's pinned staging buffer: a small solve's pageable input at 0, its
 // host output records at kTinyHostOut.
 constexpr size_t kTinyHostOut = kTinyCcMaxEdges * 8, kTinyHostBytes = kTinyHostOut + kTinyMaxVertices * 12;
 phem_status tiny_host(phem_context *ctx, char **buf);
 
 // The pointer the kernel reads a small input from: device memory of the
-// context's device in place, host memory through the pinned buffer, anything
-// else through `ws` (device workspace, `bytes` large).
+// context's device and pinned host memory in place, so in stream order like
+// everything else that earlier work on the stream may write; pageable memory
+// through the pinned buffer, unless a launch that reads the buffer may still be
+// queued (a call that timed out); anything else through `ws` (device workspace,
+// `bytes` large).
 phem_status tiny_input(phem_context *ctx, const void *p, size_t bytes, void *ws, const void **in);
 
 bool tiny_msf_fits(uint64_t m, uint64_t n);

@@ -437,3 +437,67 @@ def test_csr_pairs_at_any_offset(ctx, at, length):
     assert k.value == len(want) == length
     np.testing.assert_array_equal(got[1 + at:1 + at + length].view(np.uint64), want)
     assert (got[:1 + at] == -7).all() and (got[1 + at + length:] == -7).all()
+
+
+@pytest.mark.parametrize("call", ["msf", "cc", "canonical"])
+@pytest.mark.parametrize("n,m", [(2000, 8000), (40000, 60000)])  # one CTA, the grid
+@pytest.mark.parametrize("skip", [0, 1])
+def test_host_input_in_stream_order(ctx, call, n, m, skip):
+    """A pinned host array (at its start and 8 or 12 bytes into it) that an
+    earlier asynchronous copy on the context's stream fills is read after that
+    copy, at every size."""
+    import torch
+    pairs = gen.er(n, 2 * m, seed=n)[:m]
+    E = gen.msf_edges(pairs, gen.weights(m, m, bits=10))
+    src = E if call == "msf" else pairs
+    words = np.concatenate([src[:skip], src]).view(np.int32).reshape(-1)
+    host = torch.zeros(len(words), dtype=torch.int32).pin_memory()
+    arr = host.numpy().view(src.dtype).reshape((-1,) + src.shape[1:])[skip:]
+    stream = torch.cuda.Stream()
+    d = torch.from_numpy(words).cuda()
+    torch.cuda.synchronize()
+    ctx.set_stream(stream)
+    try:
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(20_000_000)  # about 10 ms
+            host.copy_(d, non_blocking=True)
+        if call == "msf":
+            r = ctx.msf_solve(arr, n)
+            assert_msf(r, E, *expect(E, n))
+        else:
+            r = ctx.cc_solve(arr, n, canonical=call == "canonical")
+            np.testing.assert_array_equal(r.labels, oracle.cc_solve(pairs, n)[0])
+    finally:
+        stream.synchronize()
+        ctx.set_stream(None)
+
+
+def test_pageable_input_after_a_timeout(ctx):
+    """A call that times out leaves its work to finish: a small solve from
+    pageable memory into device memory completes with its own edges although
+    the next call's are staged meanwhile."""
+    import torch
+    n = 2000
+    A, B = (gen.msf_edges(gen.er(n, 16000, seed=k)[:8000], gen.weights(8000, k, bits=10)) for k in (1, 2))
+    out = torch.zeros((n, 3), dtype=torch.int32, device="cuda")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    ctx.msf_solve(A, n, out=out)
+    out.zero_()
+    torch.cuda.synchronize()
+    ctx.set_stream(stream)
+    try:
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(100_000_000)  # about 50 ms
+        ctx.set_timeout_ms(1)
+        with pytest.raises(P.PhemError) as ei:
+            ctx.msf_solve(A, n, out=out)
+        assert ei.value.status == _lib.PHEM_ERR_TIMEOUT
+        ctx.set_timeout_ms(0)
+        assert_msf(ctx.msf_solve(B, n), B, *expect(B, n))
+        ids, cnt, _ = expect(A, n)
+        np.testing.assert_array_equal(out.cpu().numpy().view(np.uint32)[:cnt], A[ids])
+    finally:
+        ctx.set_timeout_ms(0)
+        stream.synchronize()
+        ctx.set_stream(None)
