@@ -603,7 +603,7 @@ static phem_status cc_solve_tiny(phem_context *ctx, const uint64_t *edges, int64
     const size_t o_lab = align256(eb), o_for = o_lab + align256(lb);
     PHEM_TRY(ws_reserve(ctx, o_for + align256(fb)));
     const void *in = nullptr;
-    PHEM_TRY(tiny_input(ctx, edges, eb, ctx->ws, &in));
+    PHEM_TRY(tiny_input(ctx, edges, eb, sizeof(uint64_t), ctx->ws, &in));
     Staged sl, sf;
     stage_out(ctx, labels, lb, o_lab, &sl);
     stage_out(ctx, forest, fb, o_for, &sf);
@@ -1009,7 +1009,7 @@ static phem_status msf_tiny(phem_context *ctx, const phem_edge *edges, uint64_t 
     const size_t eb = (size_t)m * sizeof(phem_edge);
     PHEM_TRY(ws_reserve(ctx, align256(eb)));
     const void *in = nullptr;
-    PHEM_TRY(tiny_input(ctx, edges, eb, ctx->ws, &in));
+    PHEM_TRY(tiny_input(ctx, edges, eb, sizeof(uint32_t), ctx->ws, &in));
     phem_edge *out = msf;
     char *host = nullptr;
     if (msf && !is_device_ptr(msf)) {

@@ -467,7 +467,7 @@ phem_status tiny_host(phem_context *ctx, char **buf)
     return PHEM_OK;
 }
 
-phem_status tiny_input(phem_context *ctx, const void *p, size_t bytes, void *ws, const void **in)
+phem_status tiny_input(phem_context *ctx, const void *p, size_t bytes, size_t word, void *ws, const void **in)
 {
     *in = p;
     if (!bytes)
@@ -477,9 +477,10 @@ phem_status tiny_input(phem_context *ctx, const void *p, size_t bytes, void *ws,
         cudaGetLastError();
         attr.type = cudaMemoryTypeUnregistered;
     }
-    if (attr.type == cudaMemoryTypeDevice && attr.device == ctx->device && ((uintptr_t)p & 3) == 0)
+    const bool fits = (uintptr_t)p % word == 0;
+    if (attr.type == cudaMemoryTypeDevice && attr.device == ctx->device && fits)
         return PHEM_OK;
-    if (attr.type == cudaMemoryTypeHost && attr.devicePointer && ((uintptr_t)p & 7) == 0) {
+    if (attr.type == cudaMemoryTypeHost && attr.devicePointer && fits) {
         *in = attr.devicePointer;
         return PHEM_OK;
     }

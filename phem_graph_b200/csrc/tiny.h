@@ -25,8 +25,9 @@ phem_status tiny_host(phem_context *ctx, char **buf);
 // everything else that earlier work on the stream may write; pageable memory
 // through the pinned buffer, unless a launch that reads the buffer may still be
 // queued (a call that timed out); anything else through `ws` (device workspace,
-// `bytes` large).
-phem_status tiny_input(phem_context *ctx, const void *p, size_t bytes, void *ws, const void **in);
+// `bytes` large).  In place only on a multiple of `word`, the kernel's narrowest
+// reads (4 bytes of {u, v, w} records, 8 of packed pairs).
+phem_status tiny_input(phem_context *ctx, const void *p, size_t bytes, size_t word, void *ws, const void **in);
 
 bool tiny_msf_fits(uint64_t m, uint64_t n);
 bool tiny_cc_fits(int64_t m, int64_t n);

@@ -394,3 +394,25 @@ def test_solves_after_failed_and_profiled_ones(ctx, n):
         np.testing.assert_array_equal(d.labels, want)
         assert d.components == c.components
         ctx.set_profiling(False)
+
+
+@pytest.mark.parametrize("where", ["device", "pinned", "pageable"])
+@pytest.mark.parametrize("m", [1, 9001, 32767, 32768, 32769])  # one CTA, and one edge more than it takes
+@pytest.mark.parametrize("words", [1, 2, 3])
+def test_pairs_at_any_word_offset(ctx, where, m, words):
+    """A pair array at every multiple of 4 bytes is solved (the small solve
+    reads packed pairs as 8-byte words; other offsets are copied first)."""
+    import torch
+    n = max(2, m // 3)
+    p = gen.er(n, 2 * m + 8, seed=m)[:m]
+    flat = np.concatenate([np.zeros(words, np.int32), p.view(np.int32)])
+    t = torch.from_numpy(flat)
+    t = t.cuda() if where == "device" else t.pin_memory() if where == "pinned" else t
+    torch.cuda.synchronize()
+    want, _ = oracle.cc_solve(p, n)
+    for flags in (0, _lib.PHEM_CC_CANONICAL):
+        lab, slots, st = np.empty(n, np.int32), np.empty(n, np.uint64), _lib.CCStats()
+        _lib.check(_lib.lib().phem_cc_solve(ctx.handle, t.data_ptr() + 4 * words, len(p), n, lab.ctypes.data,
+                                            slots.ctypes.data, flags, _lib.C.byref(st)), "phem_cc_solve")
+        np.testing.assert_array_equal(lab, want)
+        check_forest(p, n, want, slots)
