@@ -19,7 +19,8 @@
 //             root that many edges want to hook costs one CAS per CTA.  (Trying
 //             again at once with what the CAS returned read the hubs' words
 //             over and over: 851 against 384 us on R-MAT 22.)
-//   compress  the roots hooked in the round are pointed at their new roots;
+//   compress  the roots hooked in the round are pointed at their new roots
+//             (those of the last round by the passes over all vertices);
 //   the rest  a bit per vertex (in the giant component, read through L1)
 //             settles most edges; the others are gathered 32 at a time, their
 //             parents read and, where they differ, united with a CAS, as in
@@ -69,8 +70,34 @@ struct CcSmem {
     unsigned long long offered[kTriedSlots];  // vertex << 32 | smallest neighbour offered to it
     unsigned long long acc, sum;
     uint32_t abort, fatal;
-    uint32_t giant, giant_votes;
+    uint32_t giant;
 };
+
+// x to its root if that is near, for the giant component's; every block looks
+// for itself.  A last round or a rest can leave one chain of hundreds of
+// thousands of roots, whose links a walk would take one after the other while
+// the passes over all vertices shorten it from all sides: a block that finds no
+// root sets no vertex's bit, and the others' bits are still right, because a
+// root that is reached is the component's only one.
+constexpr uint32_t kNoVertex = 0xffffffffu, kGiantHops = 256;
+
+__device__ __forceinline__ bool near_root(const uint32_t *parent, uint32_t &x)
+{
+    for (uint32_t steps = 0; steps < kGiantHops; steps++) {
+        const uint32_t p = ld_par(parent + x);
+        if (p == x)
+            return true;
+        x = p;
+    }
+    return false;
+}
+
+// Steps of the rest's lockstep walks (uf.cuh), which can start on chains as long.
+// us per call without / with the bound, a path of 2^19 vertices 13 times behind a
+// component of as many: mean 1050-1870 / 113, slowest of 200 12,500 / 249 (105 as a
+// rule: most walks see the chain's links in time); a 4 x 500,000 mesh in random
+// order 224 / 230, others the same.
+constexpr uint32_t kLockstep = 64;
 
 // Four consecutive edges of tile t (zero -- a self-loop -- past `end`).
 __device__ __forceinline__ void load_edges(const unsigned long long *edges, uint64_t first, uint64_t t, uint64_t end,
@@ -185,8 +212,8 @@ __device__ __forceinline__ void cc_unite_row(const CcArgs &a, const uint2 *ring,
             }
         }
         if (on)
-            uf_unite_from(reinterpret_cast<int32_t *>(a.parent), a.forest, e, (int32_t)x, (int32_t)y, (int32_t)a.n,
-                          &a.ctl->err);
+            uf_unite_from<kLockstep>(reinterpret_cast<int32_t *>(a.parent), a.forest, e, (int32_t)x, (int32_t)y,
+                                     (int32_t)a.n, &a.ctl->err);
     }
     __syncwarp();
 }
@@ -368,25 +395,17 @@ __global__ void __launch_bounds__(kSolveThreads, 1) cc_grid_kernel(const __grid_
             uint32_t x = (lane & 1) ? (uint32_t)e : (uint32_t)(e >> 32);
             if (x >= a.n)
                 x = 0;
-            for (uint32_t steps = 0; steps <= a.n; steps++) {
-                const uint32_t p = ld_par(a.parent + x);
-                if (p == x)
-                    break;
-                x = p;
-            }
+            const bool found = __all_sync(0xffffffffu, near_root(a.parent, x));
             const unsigned peers = __match_any_sync(0xffffffffu, x);
             const uint32_t top = __reduce_max_sync(0xffffffffu, ((uint32_t)__popc(peers) << 5) | (31u - lane));
             const uint32_t root = __shfl_sync(0xffffffffu, x, 31 - (top & 31));
-            if (lane == 0) {
-                s.giant = root;
-                s.giant_votes = top >> 5;
-            }
+            if (lane == 0)
+                s.giant = found && top >> 5 >= 8 ? root : kNoVertex;
         }
         __syncthreads();
-        const bool use_giant = s.giant_votes >= 8;
-        full_compress(a.parent, a.n, nullptr, a.giant, s.giant, use_giant, &ctl->err);
+        full_compress<true>(a.parent, a.n, nullptr, a.giant, s.giant, true, &ctl->err);
         if (blockIdx.x == 0 && tid == 0)
-            ctl->misc[3] = use_giant, ctl->misc[4] = s.giant;
+            ctl->misc[3] = s.giant != kNoVertex, ctl->misc[4] = s.giant;
         if (__any_sync(0xffffffffu, bad) && lane == 0)
             set_err(&ctl->err, kErrRange);
         clock.stamp(kKCcLabel);
@@ -394,7 +413,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) cc_grid_kernel(const __grid_
     }
     if (__any_sync(0xffffffffu, bad) && lane == 0)
         set_err(&ctl->err, kErrRange);
-    full_compress(a.parent, a.n, nullptr, nullptr, 0, false, &ctl->err);
+    full_compress<true>(a.parent, a.n, nullptr, nullptr, 0, false, &ctl->err);
     count_roots(a, &s.acc);
     clock.stamp(kKCcLabel);
     publish_ctl(ctl, a.publish);
@@ -468,30 +487,40 @@ __global__ void __launch_bounds__(kRestThreads, kRestCtasPerSm) cc_rest_kernel(c
         set_err(&ctl->err, kErrRange);
 }
 
+// Blocks of the passes over all vertices: all resident at once, so that every
+// chain is shortened by its own vertices' threads while others walk it.  With
+// twice as many blocks the first ones went on to the higher vertices while the
+// last ones' vertices, which the chains lead through, had no thread yet: 19 ms for
+// a path of 2^20 vertices behind a component of as many, 0.11 now.
+constexpr int kVertexBlocksPerSm = 4;
+
 // Between two parts of the rest: every vertex to its root, and the giant
 // component's bits again (its root is looked up: it may have been hooked).
-__global__ void __launch_bounds__(kBlock) cc_regroup_kernel(const __grid_constant__ CcArgs a)
+__global__ void __launch_bounds__(kBlock, kVertexBlocksPerSm) cc_regroup_kernel(const __grid_constant__ CcArgs a)
 {
-    const bool use_giant = a.ctl->misc[3] != 0;
-    uint32_t root = (uint32_t)a.ctl->misc[4];
-    if (use_giant)
-        root = (uint32_t)uf_find<true>(reinterpret_cast<int32_t *>(a.parent), (int32_t)root, (int32_t)a.n, &a.ctl->err);
-    full_compress(a.parent, a.n, nullptr, a.giant, root, use_giant, &a.ctl->err);
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-        a.ctl->misc[5] = root;
+    __shared__ uint32_t s_giant;
+    if (threadIdx.x == 0) {
+        uint32_t root = (uint32_t)a.ctl->misc[4];
+        const bool found = a.ctl->misc[3] != 0 && near_root(a.parent, root);
+        s_giant = found ? root : kNoVertex;
+        if (blockIdx.x == 0)
+            a.ctl->misc[5] = root;  // or an ancestor of the vertices with a bit, which serves as well
+    }
+    __syncthreads();
+    full_compress<true>(a.parent, a.n, nullptr, a.giant, s_giant, true, &a.ctl->err);
 }
 
 // Labels (every vertex to its root) and the number of components.  Bound by
 // the walks' L2 latency, so by the warps in flight: two blocks per SM (102
 // registers) / four (64), us per call: n = 2^21 282 / 275, R-MAT 22 361 / 355;
 // six and eight the same as four.
-__global__ void __launch_bounds__(kBlock, 4) cc_label_count_kernel(const __grid_constant__ CcArgs a)
+__global__ void __launch_bounds__(kBlock, kVertexBlocksPerSm) cc_label_count_kernel(const __grid_constant__ CcArgs a)
 {
     __shared__ unsigned long long s_roots;
     if (threadIdx.x == 0)
         s_roots = 0;
     __syncthreads();
-    full_compress(a.parent, a.n, nullptr, nullptr, 0, false, &a.ctl->err);
+    full_compress<true>(a.parent, a.n, nullptr, nullptr, 0, false, &a.ctl->err);
     count_roots(a, &s_roots);
     publish_ctl(a.ctl, a.publish);
 }
@@ -541,7 +570,7 @@ phem_status cc_grid(phem_context *ctx, const uint64_t *d_edges, int64_t m, int64
                              ctx->stream>>>(b, part);
         };
         const int vblocks = (int)std::min<int64_t>(((int64_t)n + kBlock * kVItems - 1) / (kBlock * kVItems),
-                                                   (int64_t)ctx->sm_count * 8);
+                                                   (int64_t)ctx->sm_count * kVertexBlocksPerSm);
         // A long rest goes in two parts: the first attaches most of what the
         // prefix left out, and after a second look at the components the
         // bits settle nearly all of the second.  us per solve in one part / cut

@@ -51,15 +51,46 @@ __device__ __forceinline__ int32_t uf_find(int32_t *parent, int32_t x, int32_t n
     return x;
 }
 
+// Walks only the larger of a and b: ids fall towards the roots, so two walks up
+// one chain meet where the smaller one stands.  Returns true when they do, else
+// false with the larger one's root and an ancestor of the other that is smaller.
+__device__ __noinline__ inline bool uf_meet(int32_t *parent, int32_t a, int32_t b, int32_t n, uint32_t *err,
+                                            int32_t *ra, int32_t *rb)
+{
+    for (uint32_t steps = 0; steps <= 2 * (uint32_t)n; steps++) {
+        if (a == b)
+            return true;
+        const int32_t lo = min(a, b);
+        int32_t hi = max(a, b);
+        const int32_t p = __ldcg(parent + hi);
+        if (p == hi) {
+            *ra = hi;
+            *rb = lo;
+            return false;
+        }
+        const int32_t gp = p > lo ? __ldcg(parent + p) : p;
+        if (gp != p)
+            atomicMin(parent + hi, gp);
+        a = gp;
+        b = lo;
+    }
+    set_err(err, kErrChase);
+    *ra = a;
+    *rb = b;
+    return a == b;
+}
+
 // The roots of a and b, walked in lockstep (both walks' loads are in flight
 // together) with the same halving as uf_find.  Returns true as soon as the
 // walks meet (one component; *ra, *rb are then not set), else false with
-// the two roots.
-template <bool CACHED>
+// the two roots.  Lockstep walks that start at different heights of one chain
+// meet at its root; where chains can be long LOCKSTEP bounds their steps, and
+// uf_meet goes on (the smaller vertex returned may then have a parent).
+template <bool CACHED, uint32_t LOCKSTEP = 0>
 __device__ __forceinline__ bool uf_find2(int32_t *parent, int32_t a, int32_t b, int32_t n, uint32_t *err,
                                          int32_t *ra, int32_t *rb)
 {
-    const uint32_t cap = (uint32_t)n + 1;
+    const uint32_t cap = LOCKSTEP ? LOCKSTEP : (uint32_t)n + 1;
     bool da = false, db = false;  // walk finished at a root
     for (uint32_t steps = 0; steps < cap; steps++) {
         if (a == b)
@@ -98,6 +129,8 @@ __device__ __forceinline__ bool uf_find2(int32_t *parent, int32_t a, int32_t b, 
             b = gb;
         }
     }
+    if (LOCKSTEP)
+        return uf_meet(parent, a, b, n, err, ra, rb);
     set_err(err, kErrChase);
     *ra = a;
     *rb = b;
@@ -107,13 +140,15 @@ __device__ __forceinline__ bool uf_find2(int32_t *parent, int32_t a, int32_t b, 
 // One union with the reference's hook rule (larger root under smaller root,
 // forest[hooked root] = edge).  Returns true when it hooked.
 // u and v: the endpoints, or ancestors of theirs.
+template <uint32_t LOCKSTEP = 0>
 __device__ __forceinline__ bool uf_unite_from(int32_t *parent, unsigned long long *forest, unsigned long long e,
                                               int32_t u, int32_t v, int32_t n, uint32_t *err)
 {
     for (uint32_t retry = 0; retry < kUnionRetryCap; retry++) {
         // first attempt through L1; after a failed CAS, coherent walks
         int32_t ru, rv;
-        if (retry == 0 ? uf_find2<true>(parent, u, v, n, err, &ru, &rv) : uf_find2<false>(parent, u, v, n, err, &ru, &rv))
+        if (retry == 0 ? uf_find2<true, LOCKSTEP>(parent, u, v, n, err, &ru, &rv)
+                       : uf_find2<false, LOCKSTEP>(parent, u, v, n, err, &ru, &rv))
             return false;
         if (ru == rv)
             return false;

@@ -416,3 +416,60 @@ def test_pairs_at_any_word_offset(ctx, where, m, words):
                                             slots.ctypes.data, flags, _lib.C.byref(st)), "phem_cc_solve")
         np.testing.assert_array_equal(lab, want)
         check_forest(p, n, want, slots)
+
+
+def _zigzag(k):
+    """r_i = i, a_i = k + 2i, b_i = a_i + 1: all (r_i, a_i) and (r_i, b_i), then all (a_i, b_{i+1}).  Every vertex
+    hooks under its r_i at once, and the k roots then hook into one chain in a single round."""
+    i = np.arange(k, dtype=np.uint64)
+    a, b = np.uint64(k) + 2 * i, np.uint64(k) + 2 * i + np.uint64(1)
+    u = np.concatenate([i, i, np.minimum(a[:-1], b[1:])])
+    v = np.concatenate([a, b, np.maximum(a[:-1], b[1:])])
+    return (u << np.uint64(32)) | v, 3 * k
+
+
+def _block_and_path(n, low, repeat):
+    """n edges that make one component of n / 2 vertices, then a path over the other half in order, `repeat` times,
+    linked to the component; low: the path has the smaller ids, so the component's root ends up under it."""
+    h = n // 2
+    rng = np.random.default_rng(7)
+    x = np.concatenate([np.arange(1, h), rng.integers(1, h, n - h + 1)])
+    block = (np.zeros(n, np.uint64) << np.uint64(32)) | x.astype(np.uint64)
+    path = np.arange(h - 1, dtype=np.uint64)
+    path = (path << np.uint64(32)) | (path + np.uint64(1))
+    off = np.uint64((h << 32) | h)
+    if low:
+        block += off
+        link = np.uint64(((h - 1) << 32) | h)
+    else:
+        path += off
+        link = np.uint64((1 << 32) | h)
+    return np.concatenate([block, [link]] + [path] * repeat), n
+
+
+@pytest.mark.parametrize("kind", ["zigzag", "zigzag_rest", "path", "path_low", "path_long_rest", "path_low_long_rest",
+                                  "path_links", "path_low_links"])
+def test_chains_of_roots(ctx, kind):
+    """Roots that hook into chains of hundreds of thousands in one step, before each of the passes that point vertices
+    at their roots: labels and forest exact, and no walk of a chain one vertex after another."""
+    import torch
+    if kind.startswith("zigzag"):
+        p, n = _zigzag(350000)
+        if kind == "zigzag_rest":
+            p = np.concatenate([p, p[:n]])
+    else:
+        p, n = _block_and_path(1 << 21 if kind == "path" else 1 << 20, "low" in kind, 13 if "long" in kind else 2)
+        if "links" in kind:  # from all over the path to the other half
+            u, v = np.random.default_rng(3).integers(0, n // 2, (2, n // 4)).astype(np.uint64)
+            p = np.concatenate([p, (u << np.uint64(32)) | (v + np.uint64(n // 2))])
+    d = torch.from_numpy(p.view(np.int64)).cuda()
+    lab = torch.empty(n, dtype=torch.int32, device="cuda")
+    slots = torch.empty(n, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    ms = []
+    for _ in range(3):
+        r = ctx.cc_solve(d, n, labels=lab, forest=slots)
+        ms.append(r.device_ms)
+        assert not lab.any() and r.components == 1
+    check_forest(p, n, np.zeros(n, np.int32), slots.cpu().numpy().view(np.uint64))
+    assert min(ms) < 2.0  # 0.07 to 0.6; link by link 10 to 60
