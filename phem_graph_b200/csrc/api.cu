@@ -652,10 +652,11 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
         return cc_solve_tiny(ctx, edges, m, n, labels, forest, canonical, stats);
     const size_t eb = (size_t)m * sizeof(uint64_t), lb = (size_t)n * sizeof(int32_t),
                  fb = (size_t)n * sizeof(uint64_t);
-    // extra area: staged edges | labels | forest | parent (default path)
-    const size_t o_edges = 0, o_lab = align256(eb), o_for = o_lab + align256(lb), o_par = o_for + align256(fb);
     const bool on_device = is_device_ptr(edges);
     const bool aligned_dev = on_device && (((uintptr_t)edges & 15) == 0);
+    // extra area: staged edges (unless read in place) | labels | forest | parent (default path)
+    const size_t o_edges = 0, o_lab = aligned_dev ? 0 : align256(eb), o_for = o_lab + align256(lb),
+                 o_par = o_for + align256(fb);
     // large host inputs of the default path are copied in chunks, overlapped
     // with the unions of the chunks before them
     const bool overlap = !canonical && !on_device && m >= kOverlapMinEdges;
@@ -669,15 +670,21 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
     // prefix (a much longer one than usual stays with the launches below).  A
     // server's workers keep to the launches: they need no lists, which the
     // admission of requests does not count, and no SMs all at once (run_impl)
-    const bool one_launch = !canonical && !overlap && !ctx->shares_device && s <= 4 * (int64_t)n + (1 << 20);
-    const size_t grid_extra = o_par + (one_launch ? cc_grid_bytes(m, s, n, ctx->sm_count) : 0);
-    const size_t extra = one_launch ? grid_extra : o_par + align256(lb);
+    bool one_launch = !canonical && !overlap && !ctx->shares_device && s <= 4 * (int64_t)n + (1 << 20);
+    const size_t extra = o_par + align256(lb);
     size_t base = 0;
     MsfPlan plan;
     if (canonical) {
         PHEM_TRY(msf_plan(ctx, kKindPacked, (uint64_t)m, (uint32_t)n, extra, 0, &plan, &base));
     } else {
-        PHEM_TRY(ws_reserve(ctx, extra));
+        if (one_launch) {
+            const phem_status st = ws_reserve(ctx, o_par + cc_grid_bytes(m, s, n, ctx->sm_count));
+            one_launch = st != PHEM_ERR_NOMEM;  // else without the lists
+            if (st != PHEM_OK && one_launch)
+                return st;
+        }
+        if (!one_launch)
+            PHEM_TRY(ws_reserve(ctx, extra));
     }
     Staged se, sl, sf;
     if (aligned_dev) {

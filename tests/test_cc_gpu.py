@@ -473,3 +473,30 @@ def test_chains_of_roots(ctx, kind):
         assert not lab.any() and r.components == 1
     check_forest(p, n, np.zeros(n, np.int32), slots.cpu().numpy().view(np.uint64))
     assert min(ms) < 2.0  # 0.07 to 0.6; link by link 10 to 60
+
+
+def test_solves_without_room_for_the_lists():
+    """Device memory that holds the arrays of a solve but not the lists of the
+    one-launch form: the launches without lists solve it."""
+    import torch
+    n = 4_000_000
+    p = gen.er(n, 4_400_000, 5)
+    d = torch.from_numpy(p.view(np.int64)).cuda()
+    lab = torch.empty(n, dtype=torch.int32, device="cuda")
+    slots = torch.empty(n, dtype=torch.int64, device="cuda")
+    with P.Context(0) as c:
+        c.cc_solve(p, n)  # their kernels are loaded
+        c.trim()
+        lab.fill_(-1)
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - (100 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            r = c.cc_solve(d, n, labels=lab, forest=slots)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+    want, _ = oracle.cc_solve(p, n)
+    np.testing.assert_array_equal(lab.cpu().numpy(), want)
+    assert r.components == len(np.unique(want)) == n - r.forest_edges
+    check_forest(p, n, want, slots.cpu().numpy().view(np.uint64))
