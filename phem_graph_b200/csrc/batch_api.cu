@@ -163,16 +163,28 @@ phem_status batch_stage(phem_context *ctx, const phem_batch_graph *graphs, uint3
                         BatchGroups *grp = nullptr, BatchGrid *grid = nullptr)
 {
     PHEM_TRY(build_items(graphs, G, E, V, L));
-    const bool on_grid = grid && batch_takes_grid(*L, ctx->sm_count);
+    bool on_grid = grid && batch_takes_grid(*L, ctx->sm_count);
     if (E && !edges) {
         set_error("batch: null edge array");
         return PHEM_ERR_INVALID;
     }
     const bool dev_edges = E && is_device_ptr(edges) && ((uintptr_t)edges & 3) == 0;
-    const uint64_t wl = on_grid ? batch_grid_list(L->wl_records, G, ctx->sm_count) : L->wl_records;
-    const size_t bytes = batch_carve(G, E, wl, L->bm_words, V, !dev_edges, nullptr, nullptr);
-    PHEM_TRY(ws_reserve(ctx, on_grid ? batch_grid_carve(G, L->wl_records, V, ctx->sm_count, bytes, nullptr, nullptr)
-                                     : bytes));
+    uint64_t wl = L->wl_records;
+    size_t bytes = 0;
+    auto reserve = [&](uint64_t list) {
+        wl = list;
+        bytes = batch_carve(G, E, wl, L->bm_words, V, !dev_edges, nullptr, nullptr);
+        return ws_reserve(ctx, on_grid ? batch_grid_carve(G, L->wl_records, V, ctx->sm_count, bytes, nullptr, nullptr)
+                                       : bytes);
+    };
+    if (on_grid) {
+        const phem_status st = reserve(batch_grid_list(L->wl_records, G, ctx->sm_count));
+        on_grid = st != PHEM_ERR_NOMEM;  // else by the other kernel, which needs less
+        if (st != PHEM_OK && on_grid)
+            return st;
+    }
+    if (!on_grid)
+        PHEM_TRY(reserve(L->wl_records));
     batch_carve(G, E, wl, L->bm_words, V, !dev_edges, static_cast<char *>(ctx->ws), b);
     if (on_grid)
         batch_grid_carve(G, L->wl_records, V, ctx->sm_count, bytes, static_cast<char *>(ctx->ws), grid);

@@ -297,3 +297,30 @@ def test_plan_replays_both_kernels(ctx):
         p.run()
         with pytest.raises(PhemError):
             p.download()
+
+
+def test_large_graphs_without_room_for_the_grid():
+    """Device memory that holds a batch but not the grid kernel's arrays: the
+    CTA-per-graph kernel solves it."""
+    import phem_graph_b200 as P
+    import torch
+    n = 200000
+    p = gen.er(n, 3_000_000, 5)
+    b = gen.batch_from([("", n, gen.msf_edges(p, gen.weights(len(p), 1)), gen.PHEM_BATCH_MSF)])
+    host = b.edges
+    b.edges = torch.from_numpy(host.view(np.int32)).cuda()
+    torch.cuda.synchronize()
+    with P.Context(0) as c:
+        small = gen.mixed_batch(4, 5, 64, 300)
+        c.batch_solve(small)  # its kernel is loaded
+        c.trim()
+        torch.cuda.empty_cache()
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - (80 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            r = c.batch_solve(b)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+    flags, cnt, tot = oracle.msf_kruskal(host, n)
+    assert (int(r.count[0]), int(r.total[0])) == (cnt, tot)
+    np.testing.assert_array_equal(r.forest(b, 0), np.nonzero(flags)[0])
