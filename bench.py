@@ -390,7 +390,7 @@ def bench_batched(ctx, torch, num_graphs: int = 4096) -> dict:
             "vertices": b.total_vertices, "unit": UNIT, "value": b.total_edges / (ms / 1e3) / 1e9,
             "ms_per_batch": ms, "graphs_per_s": b.num_graphs / (ms / 1e3), "launches_per_batch": 1,
             "config": {k: tuned[k] for k in ("block_size", "items", "compact_ratio", "grid", "smem_vertices")},
-            "replay": "captured CUDA graph (both batch kernels; the one the batch is not for returns at once)",
+            "replay": "captured CUDA graph (control reset + the kernel the batch goes to)",
             "one_launch_per_graph": {"value": b.total_edges / plain_batch_s / 1e9, "s_per_batch": plain_batch_s,
                                      "sample": "256 graphs through phem_msf_solve, scaled by edge share"},
             "speedup_vs_one_launch_per_graph": plain_batch_s / (ms / 1e3),

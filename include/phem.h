@@ -390,7 +390,9 @@ phem_status phem_batch_solve(phem_context *ctx, const phem_batch_graph *graphs, 
 
 /* Replayable batch plan: device buffers sized for a maximum batch plus a
  * captured CUDA graph (queue reset + persistent kernel) that reads the batch
- * size from device memory, so one capture serves every batch that fits.
+ * size from device memory, so one capture serves every batch that fits.  The
+ * grid kernel's buffers and its captured launch are made by the first upload
+ * of a batch that goes to it.
  * Kernel configuration comes from the context's batch.* tuning at creation;
  * the context stream must not be the legacy default stream. */
 typedef struct phem_batch_plan phem_batch_plan;

@@ -58,7 +58,7 @@ struct GridItem {
     uint32_t skip;    // records between the first tile's aligned start and e_off
 };
 // Sizes of one launch of it (device memory, so one captured launch serves any
-// batch); items = 0: nothing to do.
+// batch).
 struct GridHdr {
     uint32_t items, tiles, vertices, pad;
 };
@@ -157,9 +157,17 @@ struct phem_batch_plan {
     phem::BatchBuffers buf{};
     phem::BatchLaunch launch{};
     float ratio = 0.5f;
-    phem::BatchGrid grid{};              // the grid kernel's buffers (null in a serving slot's plan)
+    // the grid kernel's part, made when a batch first goes to it
+    bool may_grid = false;               // (never in a serving slot's plan)
+    bool on_grid = false;                // the uploaded batch is the grid kernel's
+    void *grid_mem = nullptr;
+    uint4 *grid_list = nullptr;
+    phem::BatchGrid grid{};
     phem::GridItem *h_grid = nullptr;    // pinned staging of its items
     phem::GridHdr *h_hdr = nullptr;
+    float light_cc = 0.f;                // the context's tuning when the plan was made
+    cudaGraph_t grid_graph = nullptr;
+    cudaGraphExec_t grid_exec = nullptr;
     phem::BatchItem *h_items = nullptr;  // pinned staging of the work items
     uint32_t *h_num = nullptr;     // pinned batch size
     uint32_t *h_status = nullptr;  // pinned per-graph status
@@ -170,6 +178,8 @@ struct phem_batch_plan {
 };
 
 namespace phem {
+// (Re)captures the plan's CTA-per-graph launch, with `pairs` as the input of
+// kBatchPairs graphs.
 phem_status batch_plan_capture(phem_batch_plan *p, const unsigned long long *pairs);
 // phem_batch_plan_create; with `grid` the plan can also route a batch to the
 // grid kernel (a serving slot's plan cannot: its launches overlap on the

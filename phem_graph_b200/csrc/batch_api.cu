@@ -327,54 +327,78 @@ using namespace phem;
 
 namespace phem {
 
-// (Re)captures a plan's launch -- queue reset + persistent kernel -- into its
-// CUDA graph, with `pairs` as the input of kBatchPairs graphs.
-phem_status batch_plan_capture(phem_batch_plan *p, const unsigned long long *pairs)
+// Captures what `queue` puts on stream s into a graph ready to launch.
+template <class F>
+static phem_status capture_launch(cudaStream_t s, cudaGraph_t *graph, cudaGraphExec_t *exec, F queue)
 {
-    if (p->exec) {
-        cudaGraphExecDestroy(p->exec);
-        p->exec = nullptr;
-    }
-    if (p->graph) {
-        cudaGraphDestroy(p->graph);
-        p->graph = nullptr;
-    }
-    *p->h_num = 0;
-    cudaStream_t s = p->ctx->stream;
-    cudaError_t e = cudaMemcpyAsync(p->buf.num_graphs, p->h_num, sizeof(uint32_t), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess && p->grid.hdr)
-        e = cudaMemsetAsync(p->grid.hdr, 0, sizeof(GridHdr), s);
-    if (e == cudaSuccess)
-        e = cudaStreamSynchronize(s);
-    if (e == cudaSuccess)
-        e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
+    cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        const cudaError_t e1 = cudaMemsetAsync(p->buf.queue, 0, sizeof(uint32_t), s);
-        // a batch is either kernel's; the other one finds its size word zero
-        if (p->grid.hdr &&
-            batch_grid_launch(s, p->ctx->sm_count, p->grid, 0, 0, p->buf.edges, p->buf.wl,
-                              make_args(p->buf, p->buf.edges, p->ratio), kGridLightMsf,
-                              (float)p->ctx->tune_canonical_light) != PHEM_OK)
+        const bool queued = queue() == PHEM_OK;
+        e = cudaStreamEndCapture(s, graph);
+        if (e == cudaSuccess && !queued)
             e = cudaErrorUnknown;
-        BatchArgs a = make_args(p->buf, p->buf.edges, p->ratio);
-        a.pairs = pairs;
-        a.smem_vertices = p->launch.smem_vertices;
-        void *params[] = {&a};
-        const cudaError_t e2 = cudaLaunchKernel(p->launch.kernel, dim3(p->launch.grid), dim3(p->launch.block),
-                                                params, p->launch.dyn_smem, s);
-        const cudaError_t e0 = e;
-        e = cudaStreamEndCapture(s, &p->graph);
-        if (e == cudaSuccess)
-            e = e0 != cudaSuccess ? e0 : (e1 != cudaSuccess ? e1 : e2);
     }
     if (e == cudaSuccess)
-        e = cudaGraphInstantiate(&p->exec, p->graph, 0);
+        e = cudaGraphInstantiate(exec, *graph, 0);
     if (e != cudaSuccess) {
         set_error("batch plan: graph capture failed: %s", cudaGetErrorString(e));
         cudaGetLastError();
         return PHEM_ERR_CUDA;
     }
     return PHEM_OK;
+}
+
+static void drop_launch(cudaGraph_t *graph, cudaGraphExec_t *exec)
+{
+    if (*exec)
+        cudaGraphExecDestroy(*exec);
+    if (*graph)
+        cudaGraphDestroy(*graph);
+    *exec = nullptr;
+    *graph = nullptr;
+}
+
+phem_status batch_plan_capture(phem_batch_plan *p, const unsigned long long *pairs)
+{
+    drop_launch(&p->graph, &p->exec);
+    *p->h_num = 0;
+    cudaStream_t s = p->ctx->stream;
+    PHEM_CUDA_TRY(cudaMemcpyAsync(p->buf.num_graphs, p->h_num, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+    PHEM_CUDA_TRY(cudaStreamSynchronize(s));
+    return capture_launch(s, &p->graph, &p->exec, [&]() -> phem_status {
+        PHEM_CUDA_TRY(cudaMemsetAsync(p->buf.queue, 0, sizeof(uint32_t), s));
+        BatchArgs a = make_args(p->buf, p->buf.edges, p->ratio);
+        a.pairs = pairs;
+        return batch_launch(s, p->launch, a);
+    });
+}
+
+// Makes the plan's grid part (buffers for its largest batch, the captured
+// launch).  A plan of small graphs never needs it: its launch would wait for
+// every SM, and its buffers take 48 MB beside what grows with the batch.
+static phem_status plan_grid(phem_batch_plan *p)
+{
+    if (p->grid_exec)
+        return PHEM_OK;
+    const int sms = p->ctx->sm_count;
+    Carve c;
+    const size_t o_list = c.take<uint4>(batch_grid_list(p->max_wl, p->max_graphs, sms));
+    const size_t bytes = batch_grid_carve(p->max_graphs, p->max_wl, p->max_vertices, sms, c.off, nullptr, nullptr);
+    if ((!p->grid_mem && cudaMalloc(&p->grid_mem, bytes) != cudaSuccess) ||
+        (!p->h_grid && cudaMallocHost(&p->h_grid, sizeof(GridItem) * p->max_graphs) != cudaSuccess) ||
+        (!p->h_hdr && cudaMallocHost(&p->h_hdr, sizeof(GridHdr)) != cudaSuccess)) {
+        cudaGetLastError();
+        set_error("batch plan: cannot allocate %zu bytes for the grid kernel", bytes);
+        return PHEM_ERR_NOMEM;
+    }
+    char *base = static_cast<char *>(p->grid_mem);
+    p->grid_list = reinterpret_cast<uint4 *>(base + o_list);
+    batch_grid_carve(p->max_graphs, p->max_wl, p->max_vertices, sms, c.off, base, &p->grid);
+    drop_launch(&p->grid_graph, &p->grid_exec);
+    return capture_launch(p->ctx->own_stream, &p->grid_graph, &p->grid_exec, [&]() {
+        return batch_grid_launch(p->ctx->own_stream, sms, p->grid, 0, 0, p->buf.edges, p->grid_list,
+                                 make_args(p->buf, p->buf.edges, p->ratio), kGridLightMsf, p->light_cc);
+    });
 }
 
 }  // namespace phem
@@ -498,14 +522,14 @@ void phem_batch_plan_destroy(phem_batch_plan *p)
         return;
     DeviceGuard guard(p->ctx->device);
     cudaStreamSynchronize(p->ctx->stream);
-    if (p->exec)
-        cudaGraphExecDestroy(p->exec);
-    if (p->graph)
-        cudaGraphDestroy(p->graph);
+    drop_launch(&p->graph, &p->exec);
+    drop_launch(&p->grid_graph, &p->grid_exec);
     if (p->staged)
         cudaEventDestroy(p->staged);
     if (p->h_items)
         cudaFreeHost(p->h_items);
+    if (p->grid_mem)
+        cudaFree(p->grid_mem);
     if (p->h_grid)
         cudaFreeHost(p->h_grid);
     if (p->h_hdr)
@@ -551,10 +575,10 @@ phem_status phem::batch_plan_create(phem_context *ctx, uint32_t max_graphs, uint
     p->ratio = (float)ctx->tune_batch_compact;
     phem_status st = batch_launch_config(ctx->device, ctx->sm_count, ctx->tune_batch_block, ctx->tune_batch_items,
                                          &p->launch);
-    const uint64_t wl = grid ? batch_grid_list(p->max_wl, max_graphs, ctx->sm_count) : p->max_wl;
-    const size_t core = batch_carve(max_graphs, max_edges, wl, p->max_bm, max_vertices, true, nullptr, nullptr);
-    const size_t bytes =
-        grid ? batch_grid_carve(max_graphs, p->max_wl, max_vertices, ctx->sm_count, core, nullptr, nullptr) : core;
+    p->may_grid = grid;
+    p->light_cc = (float)ctx->tune_canonical_light;
+    const size_t bytes = batch_carve(max_graphs, max_edges, p->max_wl, p->max_bm, max_vertices, true, nullptr,
+                                     nullptr);
     if (st == PHEM_OK && cudaMalloc(&p->mem, bytes) != cudaSuccess) {
         cudaGetLastError();
         p->mem = nullptr;
@@ -564,18 +588,14 @@ phem_status phem::batch_plan_create(phem_context *ctx, uint32_t max_graphs, uint
     if (st == PHEM_OK && (cudaMallocHost(&p->h_items, sizeof(BatchItem) * max_graphs) != cudaSuccess ||
                           cudaMallocHost(&p->h_num, sizeof(uint32_t)) != cudaSuccess ||
                           cudaMallocHost(&p->h_status, sizeof(uint32_t) * max_graphs) != cudaSuccess ||
-                          (grid && (cudaMallocHost(&p->h_grid, sizeof(GridItem) * max_graphs) != cudaSuccess ||
-                                    cudaMallocHost(&p->h_hdr, sizeof(GridHdr)) != cudaSuccess)) ||
                           cudaEventCreateWithFlags(&p->staged, cudaEventDisableTiming) != cudaSuccess)) {
         cudaGetLastError();
         set_error("batch_plan_create: cannot allocate pinned staging");
         st = PHEM_ERR_NOMEM;
     }
     if (st == PHEM_OK) {
-        batch_carve(max_graphs, max_edges, wl, p->max_bm, max_vertices, true, static_cast<char *>(p->mem), &p->buf);
-        if (grid)
-            batch_grid_carve(max_graphs, p->max_wl, max_vertices, ctx->sm_count, core, static_cast<char *>(p->mem),
-                             &p->grid);
+        batch_carve(max_graphs, max_edges, p->max_wl, p->max_bm, max_vertices, true, static_cast<char *>(p->mem),
+                    &p->buf);
         st = phem::batch_plan_capture(p, nullptr);
     }
     if (st != PHEM_OK) {
@@ -612,20 +632,28 @@ phem_status phem_batch_plan_upload(phem_batch_plan *p, const phem_batch_graph *g
     PHEM_CUDA_TRY(cudaEventSynchronize(p->staged));  // the previous upload's staging was consumed
     std::copy(L.items.begin(), L.items.end(), p->h_items);
     // overlapping edge ranges can add up to more than the plan's edges: those
-    // batches stay with the CTA-per-graph kernel
-    const bool on_grid = p->grid.hdr && L.wl_records <= p->max_wl && batch_takes_grid(L, p->ctx->sm_count);
-    *p->h_num = on_grid ? 0 : num_graphs;
-    if (p->grid.hdr) {
-        *p->h_hdr = on_grid ? batch_grid_items(L.items.data(), num_graphs, p->h_grid) : GridHdr{};
-        PHEM_CUDA_TRY(cudaMemcpyAsync(p->grid.hdr, p->h_hdr, sizeof(GridHdr), cudaMemcpyHostToDevice, s));
-        if (on_grid)
-            PHEM_CUDA_TRY(cudaMemcpyAsync(p->grid.items, p->h_grid, sizeof(GridItem) * num_graphs,
-                                          cudaMemcpyHostToDevice, s));
+    // batches stay with the CTA-per-graph kernel, and so does every batch when
+    // there is no room for the grid's buffers
+    bool on_grid = p->may_grid && L.wl_records <= p->max_wl && batch_takes_grid(L, p->ctx->sm_count);
+    if (on_grid) {
+        const phem_status st = plan_grid(p);
+        on_grid = st != PHEM_ERR_NOMEM;
+        if (st != PHEM_OK && on_grid)
+            return st;
     }
-    if (num_graphs)
-        PHEM_CUDA_TRY(cudaMemcpyAsync(p->buf.items, p->h_items, sizeof(BatchItem) * num_graphs,
+    *p->h_num = num_graphs;
+    if (on_grid) {
+        *p->h_hdr = batch_grid_items(L.items.data(), num_graphs, p->h_grid);
+        PHEM_CUDA_TRY(cudaMemcpyAsync(p->grid.hdr, p->h_hdr, sizeof(GridHdr), cudaMemcpyHostToDevice, s));
+        PHEM_CUDA_TRY(cudaMemcpyAsync(p->grid.items, p->h_grid, sizeof(GridItem) * num_graphs,
                                       cudaMemcpyHostToDevice, s));
-    PHEM_CUDA_TRY(cudaMemcpyAsync(p->buf.num_graphs, p->h_num, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+    } else {
+        if (num_graphs)
+            PHEM_CUDA_TRY(cudaMemcpyAsync(p->buf.items, p->h_items, sizeof(BatchItem) * num_graphs,
+                                          cudaMemcpyHostToDevice, s));
+        PHEM_CUDA_TRY(cudaMemcpyAsync(p->buf.num_graphs, p->h_num, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
+    }
+    p->on_grid = on_grid;
     PHEM_CUDA_TRY(cudaEventRecord(p->staged, s));
     if (total_edges)
         PHEM_CUDA_TRY(cudaMemcpyAsync(p->buf.edges, edges, sizeof(phem_edge) * total_edges, cudaMemcpyDefault, s));
@@ -642,7 +670,7 @@ phem_status phem_batch_plan_run(phem_batch_plan *p)
     }
     DeviceGuard guard(p->ctx->device);
     p->ctx->launches[kKBatch]++;
-    PHEM_CUDA_TRY(cudaGraphLaunch(p->exec, p->ctx->stream));
+    PHEM_CUDA_TRY(cudaGraphLaunch(p->on_grid ? p->grid_exec : p->exec, p->ctx->stream));
     return PHEM_OK;
 }
 

@@ -241,8 +241,6 @@ __global__ void __launch_bounds__(kSolveThreads, 1) batch_grid_kernel(const __gr
     extern __shared__ __align__(16) unsigned char s_raw[];
     SolveSmem &s = *reinterpret_cast<SolveSmem *>(s_raw);
     const uint32_t G = a.hdr->items, T = a.hdr->tiles, V = a.hdr->vertices;
-    if (G == 0)
-        return;  // this batch is the other kernel's
     Ctl *ctl = a.s.ctl;
     const uint32_t tid = threadIdx.x, lane = lane_id(), warp = tid >> 5, nw = blockDim.x >> 5;
     uint32_t seq = 0;

@@ -324,3 +324,39 @@ def test_large_graphs_without_room_for_the_grid():
     flags, cnt, tot = oracle.msf_kruskal(host, n)
     assert (int(r.count[0]), int(r.total[0])) == (cnt, tot)
     np.testing.assert_array_equal(r.forest(b, 0), np.nonzero(flags)[0])
+
+
+def test_plan_takes_the_grid_when_needed(ctx):
+    """A plan of small graphs holds nothing for the grid kernel; a batch for
+    it gets its buffers at upload, and the other kernel while there is no room
+    for them."""
+    import torch
+    small, large = gen.mixed_batch(12, 5, 64, 300), gen.mixed_batch(6, 6, 20000, 40000)
+
+    def check(p, b):
+        p.upload(b)
+        p.run()
+        r = p.download()
+        for g in range(b.num_graphs):
+            flags, cnt, tot = oracle.msf_kruskal(b.graph_edges(g), int(b.graphs[g]["num_vertices"]))
+            assert (int(r.count[g]), int(r.total[g])) == (cnt, tot)
+            np.testing.assert_array_equal(r.forest(b, g), np.nonzero(flags)[0])
+
+    ctx.batch_solve(large)  # the kernels are loaded
+    ctx.batch_solve(small)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    with ctx.batch_plan(16, small.total_edges, small.total_vertices) as p:
+        assert free - torch.cuda.mem_get_info()[0] < 16 << 20
+        check(p, small)
+    with ctx.batch_plan(16, large.total_edges, large.total_vertices) as p:
+        check(p, small)
+        torch.cuda.empty_cache()
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - (16 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            check(p, large)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+        for b in (large, small, large):
+            check(p, b)
