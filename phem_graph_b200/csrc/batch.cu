@@ -309,8 +309,17 @@ __device__ __forceinline__ void solve_graph(const BatchArgs &a, const BatchItem 
             atomicOr(bm + (id >> 5), 1u << (id & 31));
         }
         __syncthreads();
-        // C: point every listed root at its new root, reset best, and keep the
-        // roots that had an offer and are still roots (the others are done)
+        // C: the new root of every listed root.  Set aside first: another walk's
+        // halving could still move a root's pointer back to a nearer ancestor
+        // that it had read before, and a record relabelled to that ancestor
+        // would not be offered to its component's root
+        for (uint32_t i = threadIdx.x; i < nroots; i += B) {
+            const uint32_t x = g.roots[i];
+            g.aux[x] = g_find(g.parent, x, n, &sm.err);
+        }
+        __syncthreads();
+        // every listed root at its new root, best reset, and the roots kept
+        // that had an offer and are still roots (the others are done)
         uint32_t kept = 0;
         int parity = 0;
         for (uint32_t i0 = 0; i0 < nroots; i0 += B) {
@@ -320,7 +329,7 @@ __device__ __forceinline__ void solve_graph(const BatchArgs &a, const BatchItem 
             if (i < nroots) {
                 x = g.roots[i];
                 const bool had = g.best[x] != kKeyInf;
-                const uint32_t r = g_find(g.parent, x, n, &sm.err);
+                const uint32_t r = g.aux[x];
                 if (r != x)
                     g.parent[x] = r;
                 g.best[x] = kKeyInf;

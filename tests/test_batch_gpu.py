@@ -360,3 +360,16 @@ def test_plan_takes_the_grid_when_needed(ctx):
             torch.cuda.empty_cache()
         for b in (large, small, large):
             check(p, b)
+
+
+def test_rounds_of_chains(ctx):
+    """Paths with ascending weights hook into one chain each and are done in
+    one round: every vertex's pointer is at its root when the round ends."""
+    n = 5000
+    u = np.arange(n - 1, dtype=np.uint32)
+    E = np.ascontiguousarray(np.stack([u, u + 1, u + 1], axis=1))
+    b = gen.batch_from([(f"p{i}", n, E, gen.PHEM_BATCH_MSF) for i in range(16)])
+    for _ in range(20):
+        r = ctx.batch_solve(b)
+        assert r.stats["smem_vertices"] > n and r.stats["max_rounds"] == 1
+        assert (r.count == n - 1).all() and not r.labels.any()
