@@ -320,7 +320,8 @@ def bench_batched(ctx, torch, num_graphs: int = 4096) -> dict:
     """Many small graphs: 4096 graphs, n log-uniform in [64, 65536], half
     Erdos-Renyi (mean degree U[2, 16], weights U[1, 2^20]), half 2-D random
     geometric 8-NN (weights floor(distance * 2^24)), every graph solved for
-    MSF + labels.  The autotuner picks the kernel configuration, then the
+    MSF + labels.  The autotuner picks the CTA-per-graph kernel's
+    configuration (a batch for the grid kernel does not use it), then the
     captured launch is replayed (CUDA events); the one-solve-per-launch path
     is timed on a 256-graph sample, with the inputs on the host
     (phem_msf_solve per graph) and resident on the device
@@ -389,7 +390,9 @@ def bench_batched(ctx, torch, num_graphs: int = 4096) -> dict:
     return {"workload": "batched_4096_mixed_er_rgg", "graphs": b.num_graphs, "edges": b.total_edges,
             "vertices": b.total_vertices, "unit": UNIT, "value": b.total_edges / (ms / 1e3) / 1e9,
             "ms_per_batch": ms, "graphs_per_s": b.num_graphs / (ms / 1e3), "launches_per_batch": 1,
-            "config": {k: tuned[k] for k in ("block_size", "items", "compact_ratio", "grid", "smem_vertices")},
+            "config": ({"kernel": "grid", "grid": r.stats["grid"]} if r.stats["smem_vertices"] == 0 else
+                       {"kernel": "cta_per_graph", **{k: tuned[k] for k in ("block_size", "items", "compact_ratio",
+                                                                            "grid", "smem_vertices")}}),
             "replay": "captured CUDA graph (control reset + the kernel the batch goes to)",
             "one_launch_per_graph": {"value": b.total_edges / plain_batch_s / 1e9, "s_per_batch": plain_batch_s,
                                      "sample": "256 graphs through phem_msf_solve, scaled by edge share"},

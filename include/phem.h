@@ -131,6 +131,9 @@ phem_status phem_context_launch_log(phem_context *ctx, phem_launch_record *out, 
  *   "batch.items"           records per thread per step, 1, 2 or 4         [4]
  *   "batch.compact_ratio"   a batched list pass compacts when the live
  *                           records are at most this share of the list     [1.0]
+ *   "batch.grid"            1: batches with large graphs go to the grid
+ *                           kernel, which the other batch.* keys say nothing
+ *                           about; 0: every batch to the kernel they describe [1]
  * None of them changes a result. */
 phem_status phem_context_set_tuning(phem_context *ctx, const char *key, double value);
 phem_status phem_context_get_tuning(phem_context *ctx, const char *key, double *value);
@@ -336,7 +339,7 @@ phem_status phem_csr_to_coo(phem_context *ctx, const int64_t *offsets, const uin
  * whole graphs from a device work queue (largest first) and run Boruvka on
  * each to completion; a batch whose largest graphs would keep one SM busy long
  * after the others is solved as one disjoint union by the whole grid instead
- * (the same results; the batch.* tuning then has no part).  No reference counterpart: the reference solves one
+ * (the same results; see "batch.grid").  No reference counterpart: the reference solves one
  * graph per call (boruvka_for_edge_array, MST/src/new_boruvka.cu:40-179),
  * and this is the batch of such calls without their launch overhead.  Every
  * graph gets exactly what the one-graph entry points give it:
@@ -362,12 +365,14 @@ typedef struct phem_batch_graph {
 } phem_batch_graph;
 
 typedef struct phem_batch_stats {
-    uint32_t max_rounds;    /* most Boruvka rounds any graph needed */
-    uint32_t block_size;    /* kernel configuration used */
+    uint32_t max_rounds;    /* most Boruvka rounds any graph needed (grid kernel: rounds in which any graph's
+                               components joined, light edges' and heavy edges' together) */
+    uint32_t block_size;    /* the batch.* tuning (which the grid kernel does not use) */
     uint32_t items;
     float compact_ratio;
     uint32_t grid;          /* persistent CTAs launched */
-    uint32_t smem_vertices; /* graphs up to this many vertices kept their state in shared memory */
+    uint32_t smem_vertices; /* graphs up to this many vertices kept their state in shared memory; 0: the grid
+                               kernel solved the batch */
     float device_ms;        /* GPU time of the batched launch (events on the stream) */
 } phem_batch_stats;
 
@@ -414,8 +419,9 @@ phem_status phem_batch_plan_download(phem_batch_plan *plan, uint32_t *msf_ids, u
 phem_status phem_batch_plan_device(phem_batch_plan *plan, phem_edge **edges, uint32_t **msf_ids,
                                    uint32_t **msf_count, uint64_t **msf_total, int32_t **labels);
 
-/* Autotuner: times every kernel configuration (block 256/512/1024 x items
- * 1/2/4 x compaction ratio 0.25/0.5/1.0) on this batch, `reps` launches each,
+/* Autotuner: times every configuration of the CTA-per-graph kernel (block
+ * 256/512/1024 x items 1/2/4 x compaction ratio 0.25/0.5/1.0) on this batch
+ * (whichever kernel phem_batch_solve would give it to), `reps` launches each,
  * stores the fastest in the context's batch.* tuning and reports it in
  * *best (whose device_ms is the best mean time).  Results are not returned. */
 phem_status phem_batch_autotune(phem_context *ctx, const phem_batch_graph *graphs, uint32_t num_graphs,

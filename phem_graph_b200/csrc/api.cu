@@ -475,6 +475,8 @@ phem_status phem_context_set_tuning(phem_context *ctx, const char *key, double v
         ctx->tune_batch_items = (int)value;
     } else if (k == "batch.compact_ratio" && value >= 0.0 && value <= 1.0) {
         ctx->tune_batch_compact = value;
+    } else if (k == "batch.grid" && (value == 0 || value == 1)) {
+        ctx->tune_batch_grid = (int)value;
     } else {
         set_error("set_tuning: unknown key or value out of range: %s = %g", key, value);
         return PHEM_ERR_INVALID;
@@ -512,6 +514,8 @@ phem_status phem_context_get_tuning(phem_context *ctx, const char *key, double *
         *value = ctx->tune_batch_items;
     else if (k == "batch.compact_ratio")
         *value = ctx->tune_batch_compact;
+    else if (k == "batch.grid")
+        *value = ctx->tune_batch_grid;
     else {
         set_error("get_tuning: unknown key %s", key);
         return PHEM_ERR_INVALID;

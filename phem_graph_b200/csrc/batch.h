@@ -129,8 +129,11 @@ BatchArgs make_args(const BatchBuffers &b, const phem_edge *edges, float ratio);
 
 // ---- one union over the whole grid (batch_grid.cu) ----
 constexpr float kGridLightMsf = 1.f;  // light edges per vertex of a weighted graph
-// True when the batch goes to the grid kernel.
-bool batch_takes_grid(const BatchLayout &L, int sm_count);
+// The CTAs it launches.
+uint32_t batch_grid_ctas(int sm_count);
+// True when the batch goes to the grid kernel rather than to configuration l of
+// the other one.
+bool batch_takes_grid(const BatchLayout &L, const BatchLaunch &l, int sm_count);
 // List records its survivor segments need.
 uint64_t batch_grid_list(uint64_t records, uint32_t G, int sm_count);
 // Carves its buffers behind `off` (base null: sizing only); returns the end.

@@ -160,10 +160,10 @@ phem_status batch_status(const uint32_t *status, uint32_t G)
 // left for launch_overlapped to copy.
 phem_status batch_stage(phem_context *ctx, const phem_batch_graph *graphs, uint32_t G, const phem_edge *edges,
                         uint64_t E, uint32_t V, BatchLayout *L, BatchBuffers *b, const phem_edge **d_edges,
-                        BatchGroups *grp = nullptr, BatchGrid *grid = nullptr)
+                        BatchGroups *grp = nullptr, BatchGrid *grid = nullptr, const BatchLaunch *l = nullptr)
 {
     PHEM_TRY(build_items(graphs, G, E, V, L));
-    bool on_grid = grid && batch_takes_grid(*L, ctx->sm_count);
+    bool on_grid = grid && ctx->tune_batch_grid && batch_takes_grid(*L, *l, ctx->sm_count);
     if (E && !edges) {
         set_error("batch: null edge array");
         return PHEM_ERR_INVALID;
@@ -420,9 +420,10 @@ phem_status phem_batch_solve(phem_context *ctx, const phem_batch_graph *graphs, 
     const phem_edge *d_edges = nullptr;
     BatchGroups grp;
     BatchGrid grid;
-    PHEM_TRY(batch_stage(ctx, graphs, num_graphs, edges, total_edges, total_vertices, &L, &b, &d_edges, &grp, &grid));
     BatchLaunch l;
     PHEM_TRY(batch_launch_config(ctx->device, ctx->sm_count, ctx->tune_batch_block, ctx->tune_batch_items, &l));
+    PHEM_TRY(batch_stage(ctx, graphs, num_graphs, edges, total_edges, total_vertices, &L, &b, &d_edges, &grp, &grid,
+                         &l));
     const float ratio = (float)ctx->tune_batch_compact;
     const BatchArgs args = make_args(b, d_edges, ratio);
     float ms = 0.f;
@@ -455,6 +456,10 @@ phem_status phem_batch_solve(phem_context *ctx, const phem_batch_graph *graphs, 
     }
     PHEM_TRY(stream_wait(ctx));
     PHEM_TRY(batch_status(status.data(), num_graphs));
+    if (grid.hdr) {  // what the other kernel's configuration does not say
+        l.grid = (int)batch_grid_ctas(ctx->sm_count);
+        l.smem_vertices = 0;
+    }
     fill_stats(stats, l, ratio, ms, num_graphs ? *std::max_element(rounds.begin(), rounds.end()) : 0);
     return PHEM_OK;
 }
@@ -575,7 +580,7 @@ phem_status phem::batch_plan_create(phem_context *ctx, uint32_t max_graphs, uint
     p->ratio = (float)ctx->tune_batch_compact;
     phem_status st = batch_launch_config(ctx->device, ctx->sm_count, ctx->tune_batch_block, ctx->tune_batch_items,
                                          &p->launch);
-    p->may_grid = grid;
+    p->may_grid = grid && ctx->tune_batch_grid;
     p->light_cc = (float)ctx->tune_canonical_light;
     const size_t bytes = batch_carve(max_graphs, max_edges, p->max_wl, p->max_bm, max_vertices, true, nullptr,
                                      nullptr);
@@ -634,7 +639,7 @@ phem_status phem_batch_plan_upload(phem_batch_plan *p, const phem_batch_graph *g
     // overlapping edge ranges can add up to more than the plan's edges: those
     // batches stay with the CTA-per-graph kernel, and so does every batch when
     // there is no room for the grid's buffers
-    bool on_grid = p->may_grid && L.wl_records <= p->max_wl && batch_takes_grid(L, p->ctx->sm_count);
+    bool on_grid = p->may_grid && L.wl_records <= p->max_wl && batch_takes_grid(L, p->launch, p->ctx->sm_count);
     if (on_grid) {
         const phem_status st = plan_grid(p);
         on_grid = st != PHEM_ERR_NOMEM;

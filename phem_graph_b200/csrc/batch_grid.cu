@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) batch_grid_kernel(const __gr
     if (!grid_sync(ctl, s, seq))
         return give_up();
     const bool filter = s.sum > 0;
-    uint32_t r = 0, src = kSrcLight;
+    uint32_t r = 0, joins = 0, src = kSrcLight;
     bool heavy = false;
     for (;;) {
         unsigned long long *best = a.s.best + (r & 1) * a.s.best_stride,
@@ -352,6 +352,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) batch_grid_kernel(const __gr
                 return give_up();
             compress_pass(a.s.parent, a.s.n, &ctl->err, ws);
             src = kSrcList;
+            joins++;
         } else {
             if (heavy || !filter)
                 break;
@@ -468,7 +469,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) batch_grid_kernel(const __gr
         const uint32_t nt = it.m ? (it.skip + it.m + kTileRecs - 1) / kTileRecs : 0;
         a.count[it.index] = offset(it.tile0 + nt) - offset(it.tile0);
         if (a.rounds)
-            a.rounds[it.index] = r;
+            a.rounds[it.index] = joins;  // the union's
         const uint32_t err = *(volatile uint32_t *)&ctl->err;
         if (err)
             atomicOr(a.status + it.index, err);
@@ -538,37 +539,43 @@ GridHdr batch_grid_items(const BatchItem *items, uint32_t G, GridItem *out)
 
 // Which kernel takes a batch: the one whose time, from these measured rates,
 // is shorter.  The CTA-per-graph kernel ends with its largest graph (4.5 ns per
-// edge or vertex with the state in shared memory, 10 ns without) or when its
-// two CTAs per SM have worked everything off (12 ns per edge or vertex of a
-// graph with its state in shared memory, 18 ns otherwise, 25 us per graph);
-// the grid pays its barriers once and 55 ps per edge or vertex.  us, CTA per
-// graph / grid: 256 graphs of up to 65,536 vertices (16.7 M edges and vertices)
-// 5608 / 1117, of up to 8192 566 / 353, of up to 4096 215 / 282; 4 of up to
-// 20,000 468 / 182; 2048 of up to 8192 1033 / 1144; 4096 of up to 128 451 /
-// 196, of up to 4096 1143 / 1198, of up to 16,384 3829 / 3270, of up to 65,536
-// (215 M) 15,045 / 9618.
-bool batch_takes_grid(const BatchLayout &L, int sm_count)
+// edge or vertex with the state in shared memory, 10 ns without) or when the
+// SMs have worked everything off (6 ns per SM and edge or vertex of a graph with
+// its state in shared memory, 9 ns otherwise, 12.5 us per graph); that is with
+// 1024 threads per CTA, and what 512 and 256 change is in the table.  The grid
+// pays its barriers once and 55 ps per edge or vertex.  us, CTA per graph / grid:
+// 256 graphs of up to 65,536 vertices (16.7 M edges and vertices) 5608 / 1117, of
+// up to 8192 566 / 353, of up to 4096 215 / 282; 4 of up to 20,000 468 / 182; 2048
+// of up to 8192 1033 / 1144; 4096 of up to 128 451 / 196, of up to 4096 1143 /
+// 1198, of up to 16,384 3829 / 3270, of up to 65,536 (215 M) 15,045 / 9618.  512,
+// 256 threads / grid: 256 of up to 8192 862, 1467 / 343; 2048 of up to 8192 1474,
+// 2340 / 1172; 4096 of up to 4096 889, 1294 / 1271, of up to 128 188, 115 / 203.
+bool batch_takes_grid(const BatchLayout &L, const BatchLaunch &l, int sm_count)
 {
-    constexpr uint32_t kCtaSmemVertices = 5700;  // with the default configuration
+    // one graph's time, all graphs' work and all graphs' number, against 1024 threads
+    static constexpr double kFactors[3][3] = {{1.0, 1.0, 1.0}, {1.6, 0.75, 0.27}, {2.7, 1.0, 0.06}};
+    const double *f = kFactors[l.block >= 1024 ? 0 : l.block >= 512 ? 1 : 2];
     double all = 0, cta = 0, largest = 0;
     uint64_t verts = 0;
     for (const BatchItem &x : L.items) {
         if (x.kind == kBatchPairs)
             return false;
         const double work = (double)x.m + x.n;
-        const bool smem = x.n <= kCtaSmemVertices;
+        const bool smem = x.n <= l.smem_vertices;
         all += work;
-        cta += work * (smem ? 12.0 : 18.0) + 25e3;
-        largest = std::max(largest, work * (smem ? 4.5 : 10.0));
+        cta += f[1] * work * (smem ? 6.0 : 9.0) + f[2] * 12.5e3;
+        largest = std::max(largest, f[0] * work * (smem ? 4.5 : 10.0));
         verts += ((uint64_t)x.n + 31) & ~31ull;
     }
     const uint64_t tiles = L.wl_records / kTileRecs + 2ull * L.items.size();
     if (tiles * kTileRecs >= (1ull << 32) - (1u << 24) || verts >= (1ull << 31))
         return false;  // union ids and vertices are 32-bit
-    const double cta_ns = 25e3 + std::max(largest, cta / (2.0 * sm_count));
+    const double cta_ns = 25e3 + std::max(largest, cta / sm_count);
     const double grid_ns = 190e3 + 0.055 * all;
     return grid_ns < cta_ns;
 }
+
+uint32_t batch_grid_ctas(int sm_count) { return std::min((uint32_t)sm_count, kMaxGrid); }
 
 phem_status batch_grid_launch(cudaStream_t stream, int sm_count, const BatchGrid &g, uint32_t group, uint32_t first,
                               const phem_edge *edges, uint4 *list, const BatchArgs &b, float light_msf,
@@ -603,8 +610,8 @@ phem_status batch_grid_launch(cudaStream_t stream, int sm_count, const BatchGrid
     a.light_cc = light_cc;
     PHEM_CUDA_TRY(cudaMemsetAsync(g.ctl, 0, sizeof(Ctl), stream));
     void *params[] = {&a};
-    PHEM_CUDA_TRY(cudaLaunchCooperativeKernel(batch_grid_kernel, dim3(std::min(sm_count, (int)kMaxGrid)),
-                                              dim3(kSolveThreads), params, sizeof(SolveSmem), stream));
+    PHEM_CUDA_TRY(cudaLaunchCooperativeKernel(batch_grid_kernel, dim3(batch_grid_ctas(sm_count)), dim3(kSolveThreads),
+                                              params, sizeof(SolveSmem), stream));
     return PHEM_OK;
 }
 

@@ -77,6 +77,7 @@ struct phem_context {
     int tune_batch_block = 1024;         // batched kernel: threads per CTA
     int tune_batch_items = 4;            // batched kernel: records per thread per step
     double tune_batch_compact = 1.0;     // batched kernel: compaction threshold
+    int tune_batch_grid = 1;             // large graphs as one union over the grid
     double tune_cc_sample = 1.0;         // CC: edges per vertex united before a compress (0: one pass)
     // launch accounting and optional per-kernel CUDA-event timing
     uint64_t launches[phem::kKernelCount] = {};

@@ -373,3 +373,47 @@ def test_rounds_of_chains(ctx):
         r = ctx.batch_solve(b)
         assert r.stats["smem_vertices"] > n and r.stats["max_rounds"] == 1
         assert (r.count == n - 1).all() and not r.labels.any()
+
+
+@pytest.mark.parametrize("block,items", [(256, 1), (256, 4), (512, 2), (1024, 4)])
+def test_cta_kernel_takes_every_batch_when_asked(ctx, block, items):
+    """With batch.grid 0 a batch that the grid kernel would take runs in the
+    tuned configuration, graphs above the shared-memory capacity among them,
+    through a call and through a plan."""
+    b = small_mixed(12, seed=21, n_lo=500, n_hi=40000)
+    assert ctx.batch_solve(b).stats["smem_vertices"] == 0
+    saved = [ctx.get_tuning(k) for k in TUNING]
+    try:
+        ctx.set_tuning("batch.grid", 0)
+        ctx.set_tuning("batch.block_size", block)
+        ctx.set_tuning("batch.items", items)
+        res = ctx.batch_solve(b)
+        assert 0 < res.stats["smem_vertices"] < int(b.graphs["num_vertices"].max())
+        check_batch(b, res)
+        with ctx.batch_plan(b.num_graphs, b.total_edges, b.total_vertices) as p:
+            p.upload(b)
+            p.run()
+            check_batch(b, p.download())
+    finally:
+        ctx.set_tuning("batch.grid", 1)
+        for k, v in zip(TUNING, saved):
+            ctx.set_tuning(k, v)
+
+
+@pytest.mark.parametrize("grid", [0, 1])
+def test_stats_of_both_kernels(ctx, grid):
+    """A path with ascending weights joins in one round, and so do many; the
+    statistics say which kernel ran."""
+    n = 60000
+    u = np.arange(n - 1, dtype=np.uint32)
+    b = gen.batch_from([("path", n, np.ascontiguousarray(np.stack([u, u + 1, u + 1], axis=1)), gen.PHEM_BATCH_MSF)])
+    try:
+        ctx.set_tuning("batch.grid", grid)
+        st = ctx.batch_solve(b).stats
+    finally:
+        ctx.set_tuning("batch.grid", 1)
+    assert st["max_rounds"] == 1
+    assert (st["smem_vertices"] == 0) == bool(grid) and st["device_ms"] > 0
+    if grid:
+        import torch
+        assert st["grid"] == torch.cuda.get_device_properties(0).multi_processor_count
