@@ -111,6 +111,16 @@ bool is_device_ptr(const void *p)
     return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
 }
 
+bool is_pageable(const void *p)
+{
+    cudaPointerAttributes attr;
+    if (cudaPointerGetAttributes(&attr, p) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return attr.type == cudaMemoryTypeUnregistered;
+}
+
 bool is_device_ptr_on(const void *p, int dev)
 {
     if (!p)
@@ -622,6 +632,7 @@ static phem_status cc_solve_tiny(phem_context *ctx, const uint64_t *edges, int64
                          static_cast<uint64_t *>(sf.dev)));
     }
     cudaEventRecord(ctx->ev_stop, ctx->stream);
+    PHEM_TRY(wait_before_copies(ctx, sl, sf));
     PHEM_TRY(copy_back(ctx, sl, lb));
     PHEM_TRY(copy_back(ctx, sf, fb));
     PHEM_TRY(stream_wait(ctx));
@@ -733,6 +744,7 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
     const bool counted = canonical || one_launch;
     if (!counted)
         PHEM_TRY(cc_launch_count(ctx, n, d_lab, d_for));
+    PHEM_TRY(wait_before_copies(ctx, sl, sf));
     PHEM_TRY(copy_back(ctx, sl, lb));
     PHEM_TRY(copy_back(ctx, sf, fb));
     PHEM_TRY(msf_finish(ctx, &rounds, "cc_solve"));

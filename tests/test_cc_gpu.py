@@ -500,3 +500,43 @@ def test_solves_without_room_for_the_lists():
     np.testing.assert_array_equal(lab.cpu().numpy(), want)
     assert r.components == len(np.unique(want)) == n - r.forest_edges
     check_forest(p, n, want, slots.cpu().numpy().view(np.uint64))
+
+
+@pytest.mark.parametrize("n,m", [(3000, 9000), (40000, 200000)])  # one CTA, the grid
+@pytest.mark.parametrize("canonical", [False, True])
+def test_pageable_outputs_do_not_hold_up_other_threads(ctx, n, m, canonical):
+    """While one thread waits for a solve with results in pageable memory,
+    behind other work on its stream, another thread's solves on a context of
+    its own go on."""
+    import threading
+    import time
+    import torch
+    p, q = gen.er(n, m, 3), gen.er(2000, 8000, 4)
+    d, dq = (torch.from_numpy(x.view(np.int64)).cuda() for x in (p, q))
+    ahead = torch.zeros(1 << 26, device="cuda")
+    stream = torch.cuda.Stream()
+    out = {}
+
+    def solve():
+        ctx.set_stream(stream)
+        out["r"] = ctx.cc_solve(d, n, canonical=canonical)
+        ctx.set_stream(None)
+
+    with P.Context(0) as other:
+        solve()
+        other.cc_solve(dq, 2000)
+        ahead.add_(1)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            for _ in range(800):  # about 0.07 s of kernels
+                ahead.add_(1)
+        t = threading.Thread(target=solve)
+        t.start()
+        calls = []
+        while t.is_alive():
+            t0 = time.perf_counter()
+            other.cc_solve(dq, 2000)
+            calls.append(time.perf_counter() - t0)
+        t.join()
+    np.testing.assert_array_equal(out["r"].labels, oracle.cc_solve(p, n)[0])
+    assert len(calls) > 20 and max(calls) < 0.02
