@@ -60,13 +60,6 @@ enum : uint32_t {
 };
 
 // ---------------------------------------------------------------- memory helpers
-__device__ __forceinline__ uint32_t ld_cg(const uint32_t *p) { return __ldcg(p); }
-__device__ __forceinline__ int32_t ld_cg(const int32_t *p) { return __ldcg(p); }
-__device__ __forceinline__ uint64_t ld_cg(const uint64_t *p)
-{
-    return (uint64_t)__ldcg(reinterpret_cast<const unsigned long long *>(p));
-}
-
 __device__ __forceinline__ uint64_t ld_relaxed_u64(const uint64_t *p)
 {
     uint64_t v;
@@ -206,9 +199,6 @@ __device__ __forceinline__ uint32_t lookback_exclusive(uint64_t *status, uint32_
     return lookback_resolve(status, tile, agg, epoch, err);
 }
 
-// Grid size for the persistent streaming kernels: whole waves over 148 SMs.
-inline int persistent_blocks(int sm_count, int blocks_per_sm) { return sm_count * blocks_per_sm; }
-
 // ---------------------------------------------------------------- bulk copies (TMA, sm_90+)
 // 1-D cp.async.bulk global -> shared with mbarrier completion.  Plain loads
 // only: no cluster multicast anywhere in this library.
@@ -234,15 +224,6 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t *bar, uint32_t by
                  : "memory");
 }
 
-// dst, src 16-byte aligned; bytes a multiple of 16.
-__device__ __forceinline__ void bulk_copy_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                     smem_addr(dst)),
-                 "l"(src), "r"(bytes), "r"(smem_addr(bar))
-                 : "memory");
-}
-
 // L2 policy for data read once (streamed inputs): evict first, so the
 // streams do not push small, reused arrays (parent, best) out of L2.
 __device__ __forceinline__ uint64_t l2_evict_first()
@@ -252,7 +233,7 @@ __device__ __forceinline__ uint64_t l2_evict_first()
     return policy;
 }
 
-// bulk_copy_g2s with an L2 cache policy for the source.
+// dst, src 16-byte aligned; bytes a multiple of 16; `policy`: an L2 cache policy for the source.
 __device__ __forceinline__ void bulk_copy_g2s_hint(void *dst, const void *src, uint32_t bytes, uint64_t *bar,
                                                    uint64_t policy)
 {
