@@ -501,3 +501,22 @@ def test_pageable_input_after_a_timeout(ctx):
         ctx.set_timeout_ms(0)
         stream.synchronize()
         ctx.set_stream(None)
+
+
+@pytest.mark.parametrize("n,m", [(1500, 8000), (20000, 100003), (60000, 230001)])
+def test_rounds_of_an_unfiltered_solve(ctx, n, m):
+    """Below the filter's size a solve is plain Boruvka: the edges and the
+    components of each round are the oracle's, in one CTA and on the grid; the
+    keys of the former round loops still round-trip."""
+    pairs = gen.er(n, m + m // 8, seed=m)[:m]
+    E = gen.msf_edges(pairs, gen.weights(len(pairs), m))
+    _, _, _, m_r, n_r = oracle.msf_boruvka(E, n)
+    r = ctx.msf_solve(E, n)
+    k = len(m_r)
+    assert r.rounds in (k, k + 1) and r.m_r[:k] == [int(x) for x in m_r] and r.n_r[:k] == [int(x) for x in n_r]
+    assert not any(r.m_r[k:])
+    for key, value in (("msf.first_batch", 9), ("msf.next_batch", 2), ("msf.graph", 0)):
+        old = ctx.get_tuning(key)
+        ctx.set_tuning(key, value)
+        assert ctx.get_tuning(key) == value
+        ctx.set_tuning(key, old)
