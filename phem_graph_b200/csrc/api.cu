@@ -207,18 +207,21 @@ phem_status status_reserve(phem_context *ctx, size_t words)
 
 phem_status stream_wait(phem_context *ctx)
 {
-    if (!ctx->timeout_ms) {
-        PHEM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    auto done = [ctx] {
+        if (ctx->tiny_busy == ctx->stream)
+            ctx->tiny_busy = nullptr;
         resolve_timings(ctx);
         return PHEM_OK;
+    };
+    if (!ctx->timeout_ms) {
+        PHEM_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+        return done();
     }
     const auto deadline = std::chrono::steady_clock::now() + std::chrono::milliseconds(ctx->timeout_ms);
     for (;;) {
         cudaError_t e = cudaStreamQuery(ctx->stream);
-        if (e == cudaSuccess) {
-            resolve_timings(ctx);
-            return PHEM_OK;
-        }
+        if (e == cudaSuccess)
+            return done();
         if (e != cudaErrorNotReady) {
             set_error("stream: %s", cudaGetErrorString(e));
             return PHEM_ERR_CUDA;

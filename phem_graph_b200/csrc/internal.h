@@ -60,6 +60,7 @@ struct phem_context {
     bool solve_ctl_zero = false;       // ... the last one zeroed it
     bool publishes = false;            // the queued solve does
     void *tiny_host = nullptr;         // pinned staging of small host solves (tiny.cu), made on first use
+    cudaStream_t tiny_busy = nullptr;  // the stream of the launch that reads it, until that has been waited for
     uint32_t tiny_ready = 0;           // bit k: launch attributes of small-solve kernel k are set
     uint64_t epoch = 1;                // look-back epoch counter
     uint32_t timeout_ms = 0;

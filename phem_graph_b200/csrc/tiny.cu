@@ -484,14 +484,14 @@ phem_status tiny_input(phem_context *ctx, const void *p, size_t bytes, size_t wo
         *in = attr.devicePointer;
         return PHEM_OK;
     }
-    if (attr.type == cudaMemoryTypeUnregistered && cudaStreamQuery(ctx->stream) == cudaSuccess) {
+    if (attr.type == cudaMemoryTypeUnregistered && !ctx->tiny_busy) {
         char *buf = nullptr;
         PHEM_TRY(tiny_host(ctx, &buf));
         std::memcpy(buf, p, bytes);
+        ctx->tiny_busy = ctx->stream;
         *in = buf;
         return PHEM_OK;
     }
-    cudaGetLastError();  // "not ready" is no error
     *in = ws;
     PHEM_CUDA_TRY(cudaMemcpyAsync(ws, p, bytes, cudaMemcpyDefault, ctx->stream));
     return PHEM_OK;
