@@ -18,7 +18,12 @@
  * are never copied.
  *
  * Streams.  All GPU work of a context is ordered on its stream.  Entry points
- * return after the work is complete unless they say "asynchronous".
+ * return after the work is complete unless they say "asynchronous".  Solves and
+ * batches past the sizes that one CTA takes are cooperative launches with a CTA
+ * on every SM: one starts when every SM has room for it.  Kernels of other
+ * streams that come and go only delay it; a kernel that stays on an SM (one that
+ * polls, or a collective that waits for a peer) delays it until that kernel
+ * ends, so such a kernel must not wait for the solve.
  *
  * Errors.  A non-zero phem_status is returned; phem_last_error() gives a
  * one-line description (thread-local).  Device loops are bounded: a loop that

@@ -28,9 +28,12 @@
 // The labels array is the parent array: the last compress leaves the labels.
 //
 // us per call, before (cc.cu's launches) -> now: uniform n = 2,000,003, m = 2^23
-// 450 -> 275, R-MAT 22 (67 M edges) 444 -> 355.  Bound: the rest's gathers and
+// 450 -> 273, R-MAT 22 (67 M edges) 444 -> 348.  Bound: the rest's gathers and
 // bits (64% L1 hits, 47% of the L2 sector rate, 56% of the issue slots on R-MAT
-// 21) and, for uniform graphs, the scattered accesses of the rounds.
+// 21) and, for uniform graphs, the scattered accesses of the rounds.  Slower than
+// before where no giant component forms and the rest still unites much: a mesh of
+// 4 x 500,000 in random order 207 -> 228 (its rest 54 -> 80, with 32 warps per SM
+// against 60; three blocks per SM 218, but geometric n = 2^19 178 -> 200).
 #include <algorithm>
 
 #include "solve.cuh"

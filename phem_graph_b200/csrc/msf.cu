@@ -728,11 +728,10 @@ phem_status run_impl(phem_context *ctx, MsfPlan &plan)
     a.threshold = k && KIND == kKindPacked ? k : kKeyNone;
     a.nsamp = k && KIND == kKindMsf ? sample_count(plan.m) : 0;
     constexpr uint32_t rec_bytes = KIND == kKindMsf ? 12 : 8;
-    // a cooperative launch waits until all its CTAs fit at once, and behind a
-    // server's batch launches half of the SMs are free sooner: mixed requests
-    // at saturation 1.92 Gedges/s with all SMs and the one-launch CC, 1.96 with
-    // half of them and cc.cu's launches (MSF as a launch per phase 1.97 to
-    // 2.03), p50 at 1,000 requests/s 1.80 / 1.65 ms (1.72)
+    // a cooperative launch waits until all its CTAs fit at once, and beside a
+    // server's other work half of the SMs are free sooner and leave the rest to
+    // it: mixed requests at saturation 3026 per second with all SMs, 3057 with
+    // half of them (MSF as a launch per phase 2936)
     const int sms = ctx->shares_device ? std::max(1, ctx->sm_count / 2) : ctx->sm_count;
     const SolveGrid g = solve_grid(plan.m, rec_bytes, sms, ctx->tune_edge_ctas);
     a.seg = seg_records(plan.m, g.blocks * (uint32_t)(g.threads / 32), rec_bytes);

@@ -7,8 +7,8 @@
 // k * 1024 + thread, so its id is implied and a record never moves), and the
 // per-vertex state lives in shared memory.  Host inputs are read in place from
 // pinned memory (the caller's, or staging for a pageable array) and results are
-// written to it, so a host call queues no copy of its own; the control block's results go straight to its
-// pinned mirror.
+// written to it, so a host call queues no copy of its own; the control block's
+// results go straight to its pinned mirror.
 //
 // Bound: shared-memory gathers.  A live record costs four per round (its two
 // parents, their best weights), about four cycles a warp each with random
