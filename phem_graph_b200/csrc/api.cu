@@ -672,7 +672,8 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
                  fb = (size_t)n * sizeof(uint64_t);
     const bool on_device = is_device_ptr(edges);
     const bool aligned_dev = on_device && (((uintptr_t)edges & 15) == 0);
-    // extra area: staged edges (unless read in place) | labels | forest | parent (default path)
+    // extra area: staged edges (unless read in place) | labels | forest | parent (default path; the
+    // canonical solve has its own)
     const size_t o_edges = 0, o_lab = aligned_dev ? 0 : align256(eb), o_for = o_lab + align256(lb),
                  o_par = o_for + align256(fb);
     // large host inputs of the default path are copied in chunks, overlapped
@@ -689,7 +690,7 @@ phem_status phem_cc_solve(phem_context *ctx, const uint64_t *edges, int64_t m, i
     // server's workers keep to the launches: they need no lists, which the
     // admission of requests does not count, and no SMs all at once (run_impl)
     bool one_launch = !canonical && !overlap && !ctx->shares_device && s <= 4 * (int64_t)n + (1 << 20);
-    const size_t extra = o_par + align256(lb);
+    const size_t extra = o_par + (canonical ? 0 : align256(lb));
     size_t base = 0;
     MsfPlan plan;
     if (canonical) {

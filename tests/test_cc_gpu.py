@@ -502,6 +502,29 @@ def test_solves_without_room_for_the_lists():
     check_forest(p, n, want, slots.cpu().numpy().view(np.uint64))
 
 
+def test_canonical_solve_of_many_vertices_in_little_memory():
+    """The canonical forest of 8,000,000 vertices and few edges, results on
+    the host, in 290 MB of device memory (it needs 32 bytes per vertex)."""
+    import torch
+    n = 8_000_000
+    p = gen.er(n, 100_000, 5)
+    with P.Context(0) as c:
+        want = c.cc_solve(p, n, canonical=True)
+        c.trim()
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - (290 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            r = c.cc_solve(p, n, canonical=True)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+    labels, forest = oracle.cc_solve(p, n)
+    for x in (want, r):
+        np.testing.assert_array_equal(x.labels, labels)
+        np.testing.assert_array_equal(forest_set(x.forest), oracle.forest_set(forest))
+
+
 @pytest.mark.parametrize("n,m", [(3000, 9000), (40000, 200000)])  # one CTA, the grid
 @pytest.mark.parametrize("canonical", [False, True])
 def test_pageable_outputs_do_not_hold_up_other_threads(ctx, n, m, canonical):
