@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) batch_grid_kernel(const __gr
     if (!grid_sync(ctl, s, seq))
         return give_up();
     const bool filter = s.sum > 0;
-    uint32_t r = 0, joins = 0, src = kSrcLight;
+    uint32_t r = 0, src = kSrcLight;
     bool heavy = false;
     for (;;) {
         unsigned long long *best = a.s.best + (r & 1) * a.s.best_stride,
@@ -352,7 +352,6 @@ __global__ void __launch_bounds__(kSolveThreads, 1) batch_grid_kernel(const __gr
                 return give_up();
             compress_pass(a.s.parent, a.s.n, &ctl->err, ws);
             src = kSrcList;
-            joins++;
         } else {
             if (heavy || !filter)
                 break;
@@ -469,7 +468,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) batch_grid_kernel(const __gr
         const uint32_t nt = it.m ? (it.skip + it.m + kTileRecs - 1) / kTileRecs : 0;
         a.count[it.index] = offset(it.tile0 + nt) - offset(it.tile0);
         if (a.rounds)
-            a.rounds[it.index] = joins;  // the union's
+            a.rounds[it.index] = r - 1 - (uint32_t)heavy;  // the union's; a phase ends with an empty pass
         const uint32_t err = *(volatile uint32_t *)&ctl->err;
         if (err)
             atomicOr(a.status + it.index, err);
