@@ -210,6 +210,8 @@ phem_status stream_wait(phem_context *ctx)
     auto done = [ctx] {
         if (ctx->tiny_busy == ctx->stream)
             ctx->tiny_busy = nullptr;
+        if (ctx->unfinished == ctx->stream)
+            ctx->unfinished = nullptr;
         resolve_timings(ctx);
         return PHEM_OK;
     };
@@ -228,6 +230,7 @@ phem_status stream_wait(phem_context *ctx)
         }
         if (std::chrono::steady_clock::now() > deadline) {
             set_error("watchdog: work not finished after %u ms", ctx->timeout_ms);
+            ctx->unfinished = ctx->stream;
             return PHEM_ERR_TIMEOUT;
         }
         std::this_thread::sleep_for(std::chrono::microseconds(50));

@@ -59,6 +59,7 @@ struct phem_context {
     phem::Ctl *solve_ctl = nullptr;    // control block of solves that publish their results themselves
     bool solve_ctl_zero = false;       // ... the last one zeroed it
     bool publishes = false;            // the queued solve does
+    cudaStream_t unfinished = nullptr; // where a call timed out: its solve may still publish
     void *tiny_host = nullptr;         // pinned staging of small host solves (tiny.cu), made on first use
     cudaStream_t tiny_busy = nullptr;  // the stream of the launch that reads it, until that has been waited for
     uint32_t tiny_ready = 0;           // bit k: launch attributes of small-solve kernel k are set

@@ -761,7 +761,9 @@ uint64_t list_capacity(uint64_t m, int sm_count)
 
 phem_status solve_ctl(phem_context *ctx, Ctl **ctl, Ctl **publish)
 {
-    ctx->publishes = !ctx->profiling;  // a profiled solve's time stamps stay in the block
+    // a profiled solve's time stamps stay in the block; and behind a solve that
+    // may still publish its own results, these are copied after it
+    ctx->publishes = !ctx->profiling && !ctx->unfinished;
     *ctl = ctx->publishes ? ctx->solve_ctl : ctx->ctl;
     *publish = ctx->publishes ? ctx->h_ctl : nullptr;
     if (!ctx->publishes || !ctx->solve_ctl_zero)

@@ -503,6 +503,38 @@ def test_pageable_input_after_a_timeout(ctx):
         ctx.set_stream(None)
 
 
+def test_grid_solves_after_a_timeout(ctx):
+    """Behind a solve that a timed-out call left on the stream, the next calls
+    return their own results, and the first one's output is completed."""
+    import torch
+    n = 40000
+    A, B = (gen.msf_edges(gen.er(n, 400000, seed=k)[:200000], gen.weights(200000, k, bits=10)) for k in (1, 2))
+    dA = torch.from_numpy(A.view(np.int32)).cuda()
+    out = torch.zeros((n, 3), dtype=torch.int32, device="cuda")
+    pairs = gen.er(n, 60000, seed=3)
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    ctx.msf_solve(B, n)
+    ctx.set_stream(stream)
+    try:
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(100_000_000)  # about 50 ms
+        ctx.set_timeout_ms(1)
+        with pytest.raises(P.PhemError) as ei:
+            ctx.msf_solve_device(dA, len(A), n, out)
+        assert ei.value.status == _lib.PHEM_ERR_TIMEOUT
+        ctx.set_timeout_ms(0)
+        assert_msf(ctx.msf_solve(B, n), B, *expect(B, n))
+        np.testing.assert_array_equal(ctx.cc_solve(pairs, n).labels, oracle.cc_solve(pairs, n)[0])
+        assert_msf(ctx.msf_solve(A, n), A, *expect(A, n))
+        ids, cnt, _ = expect(A, n)
+        np.testing.assert_array_equal(out.cpu().numpy().view(np.uint32)[:cnt], A[ids])
+    finally:
+        ctx.set_timeout_ms(0)
+        stream.synchronize()
+        ctx.set_stream(None)
+
+
 @pytest.mark.parametrize("n,m", [(1500, 8000), (20000, 100003), (60000, 230001)])
 def test_rounds_of_an_unfiltered_solve(ctx, n, m):
     """Below the filter's size a solve is plain Boruvka: the edges and the
